@@ -28,8 +28,8 @@ NEUMANN, DIRICHLET, FREESLIP = 0, 1, 2
 
 
 def build() -> bool:
-    """Build the library from the reference tree when that tree is present. Returns whether it exists."""
-    if os.path.isdir(_REF_TREE):
+    """Build the library from the reference tree when its sources are there. Returns whether it exists."""
+    if os.path.isdir(os.path.join(_REF_TREE, "src", "terra")):
         subprocess.run(["make", "-s", "-j8", "-C", os.path.join(_HERE, "ref"), "REF=" + _REF_TREE], check=True)
     return os.path.exists(_LIB_PATH)
 
