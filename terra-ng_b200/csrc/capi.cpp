@@ -86,6 +86,7 @@ void init_edd(tn::EpsDivDivOp& e, tn::Shell* sh, int level, int precision, const
     e.k.alloc(n * es);
     tn::cuda_check(cudaMemcpy(e.k.get(), e.q0 ? k_cell_dev : k_nodal_dev, n * es, cudaMemcpyDeviceToDevice),
                    "copy coefficient");
+    e.prepare_boundary(nullptr);
 }
 
 template <typename Op>

@@ -11,26 +11,44 @@
 // with M = [p1-p0, p2-p0, (p0+p1+p2)/3] built from unit-sphere corners only
 // (kernel_helpers.hpp:179-258). With M^{-T} = [e1 e2 e3] the physical gradient
 // of node (m, side s) is g = alpha L_m + s beta e3, alpha = 1/(2 r_mid),
-// beta = 1/(3 dr), L_1 = e1, L_2 = e2, L_0 = -(e1 + e2). The velocity gradient
-// of a wedge is then G = e1 (x) a + e2 (x) b + e3 (x) D (alpha, beta folded in),
-// the stress sigma = k|det J| (2 sym G - 2/3 tr G I), and the nodal outputs
-// sigma g. About 110 flops per wedge instead of two 3x3 inversions plus the
-// per-node gather/scatter of the reference.
+// beta = 1/(3 dr), L_1 = e1, L_2 = e2, L_0 = -(e1 + e2). With the corner sums
+// S = u_top + u_bot and differences D = u_top - u_bot the velocity gradient is
+//   G / alpha = e1 (x) (S1 - S0) + e2 (x) (S2 - S0) + e3 (x) rho (D0 + D1 + D2),
+// rho = beta / alpha, and the nodal forces are sigma g. Two scalings move out of
+// the wedge loop: sqrt|det M| goes into the lateral vectors (g_i = sqrt|det M| e_i,
+// a table per level), and alpha^2 r_mid^2 dr/2 = dr/8 goes into the coefficient.
+// A wedge is then 65 multiply-adds on nine lateral numbers: symmetric gradient 27,
+// stress 11, sigma g_i 27.
 //
-// Work decomposition (one CTA = a tile of TY node lines in y x a chunk of CX
-// node rows in x x all radial nodes of one diamond):
-//   * lanes run along r (CPL consecutive radial cells per lane): coalesced
-//     access to the r-fastest layout, radial node sums by warp shuffles;
-//   * warp w owns cell strip y = y0 - 1 + w; strip-to-strip sums go through
-//     shared memory, the strip left of the tile is recomputed (halo);
-//   * the CTA sweeps x; the two cell columns that meet at a node row are
-//     consecutive steps, so x sums are carried in registers;
-//   * each new node row (TY + 2 columns x nr values, contiguous in global
-//     memory) is staged by one TMA bulk copy per field into a 3-deep ring,
-//     two rows ahead of use. Every node value is written once by its owner:
-//     no atomics, no zeroing pass.
-// Diamond-edge duplicates hold this diamond's partial sums afterwards; the
-// interface-sum kernel completes them.
+// Every corner collects a lateral part L = sum sigma g_1,2 and a radial part
+// R = sum sigma g_3 over the cells around its node line; only the sums are turned
+// into node values, bottom = L - rho R and top = L + rho R. So the lateral sums
+// run on six numbers per (node line, radial cell) and the radial neighbours meet
+// once per node (three shuffles) instead of once per cell corner (twelve).
+//
+// Work decomposition:
+//   * one cell per lane, lanes along r. A cell strip (fixed y) of nrc radial cells takes nrc / 32 warps ("chunks"), or,
+//     below 32 radial cells, several strips share a warp.
+//   * a CTA owns ty node lines (ty + 1 strips: the one left of the tile is recomputed) and sweeps x. Sums between strips
+//     go through shared memory, one barrier a row; the column behind is kept in registers, inputs (S, D, k) as well as
+//     outputs (L, R), so each row is read from shared memory once.
+//   * the sweep is flattened over all tiles: CTA b takes rows [b n, (b + 1) n) of the sequence (diamond, tile, x), so all
+//     SMs finish together; only the first row of a range repeats a cell column.
+//   * two more warps stage: one issues the TMA bulk copies (no multicast) of whole rows and of the strips' geometry into
+//     a 6-deep ring, the other applies the input side of the boundary treatment to the two boundary node planes in
+//     shared memory, two rows ahead of use, and leaves the output-side record of each boundary node (normal and
+//     Ann (n.u), or diag u). So the compute warps treat a boundary node with one add. The diagonals of the boundary
+//     rows come from a table built with the operator.
+// Every node value is written once by its owner: no atomics, no zeroing pass.
+// Diamond-edge duplicates hold this diamond's partial sums afterwards; the interface-sum kernel completes them.
+//
+// What bounds it: issue, at 420 (FP32) and 480 (FP64) warp instructions per row, half of them floating point. With
+// radial sums per cell corner, radial factors and boundary code in every lane and a chunked grid the same apply took
+// 820 / 1070 instructions per cell. Measured on the level-6 apply with interface sum (L2 flushed): FP32 115 -> 69 us,
+// FP64 199 -> 102 us; level 7, FP64, per-cell coefficient: 1291 -> 703 us. Tried and slower: FP32 pairs on the
+// packed FP32x2 instructions (12 warps of 152 registers: half the instructions per cell, but 0.48 instead of 0.70
+// issue; 71 us), mbarriers between neighbouring warps instead of the row barrier (79 us FP32, 126 us FP64),
+// 14 FP64 warps of 128 registers (116 us), 20 FP32 warps of 80 registers (71 us).
 #include "tn_device.cuh"
 #include "tn_kernels.hpp"
 #include "tn_wedge_math.cuh"
@@ -43,567 +61,733 @@
 namespace tn {
 namespace {
 
-// Warps per CTA (tile_y + 1): FP64 needs up to 255 registers per thread (8
-// warps fill the register file), FP32 fits 12 warps.
-// devices a process can drive (per-device launch caches)
-constexpr int kMaxDevices = 64;
+constexpr int kMaxDevices = 64;  // devices a process can drive (per-device launch caches)
 
+// Block shape per precision. FP32: 24 compute warps at 72 registers (six a scheduler). FP64: three warpgroups of
+// compute warps and one for staging; launched with 128 registers a thread, the compute warpgroups grow to 152 out of
+// what the staging warpgroup gives up (3 x 152 + 56 = 4 x 128, so no more is asked for than the block holds).
 template <typename T>
-struct MaxWarps;
+struct Shape;
 template <>
-struct MaxWarps<double> {
-    static constexpr int value = 8;
+struct Shape<double> {
+    static constexpr int  kComputeWarps = 12, kThreads = 512, kGeo = 20;
+    static constexpr bool kSplit        = true;
+    static constexpr int  kComputeRegs = 152, kStageRegs = 56;
+    static_assert(3 * kComputeRegs + kStageRegs <= 4 * 128, "register split");
 };
 template <>
-struct MaxWarps<float> {
-    static constexpr int value = 12;
+struct Shape<float> {
+    static constexpr int  kComputeWarps = 24, kThreads = 896, kGeo = 24;
+    static constexpr bool kSplit        = false;
+    static constexpr int  kComputeRegs = 72, kStageRegs = 72;
 };
-
-// ---------------------------------------------------------------------------
-// FP32 interior cells two at a time. A lane's radial cells c and c + 32 share
-// their lateral geometry, so the arithmetic of hex_interior runs on float2
-// pairs with the packed FP32 instructions of sm_100 (FFMA2 / FADD2 / FMUL2):
-// one instruction per two cells. Subtraction is fma(b, -1, a), which rounds
-// like a - b. The nodal outputs are assembled per corner: corners 0 and 3
-// belong to one wedge each, corners 1 and 2 to both, with the lateral part
-// lat and radial part rad giving bottom = lat - rad and top = lat + rad.
-// ---------------------------------------------------------------------------
-using f2 = float2;
-__device__ __forceinline__ f2 p_add(f2 a, f2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ f2 p_sub(f2 a, f2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
-__device__ __forceinline__ f2 p_mul(f2 a, f2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ f2 p_fma(f2 a, f2 b, f2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ f2 p_bc(float a) { return make_float2(a, a); }
-
-__device__ __forceinline__ void hex_interior_x2(const f2 (&u)[4][2][3], const f2 (&ks)[4], f2 kcell, bool q0,
-                                                const float* geo, f2 alpha, f2 beta, f2 dfac, f2 (&out)[4][2][3])
-{
-    f2 S[4][3], Dq[4][3];
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            S[q][c]  = p_add(u[q][0][c], u[q][1][c]);
-            Dq[q][c] = p_sub(u[q][1][c], u[q][0][c]);
-        }
-    f2 v1w[2][3], v2w[2][3], wvw[2][3];
-#pragma unroll
-    for (int w = 0; w < 2; ++w) {
-        const float* gw  = geo + 10 * w;
-        const int    q0i = wedge_corner(w, 0), q1i = wedge_corner(w, 1), q2i = wedge_corner(w, 2);
-        const f2     kv  = q0 ? kcell : p_add(p_add(ks[q0i], ks[q1i]), ks[q2i]);
-        const f2     kw  = p_mul(kv, p_mul(dfac, p_bc(gw[9])));
-        f2           E1[3], E2[3], E3[3], a[3], b[3], D[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            E1[i] = p_mul(alpha, p_bc(gw[i]));
-            E2[i] = p_mul(alpha, p_bc(gw[3 + i]));
-            E3[i] = p_mul(beta, p_bc(gw[6 + i]));
-            a[i]  = p_sub(S[q1i][i], S[q0i][i]);
-            b[i]  = p_sub(S[q2i][i], S[q0i][i]);
-            D[i]  = p_add(p_add(Dq[q0i][i], Dq[q1i][i]), Dq[q2i][i]);
-        }
-        f2 gd[3], h[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) gd[i] = p_fma(E3[i], D[i], p_fma(E2[i], b[i], p_mul(E1[i], a[i])));
-        // h[k] for the pair (i, j) = (0,1), (0,2), (1,2)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;
-            f2        t = p_mul(E1[i], a[j]);
-            t           = p_fma(E1[j], a[i], t);
-            t           = p_fma(E2[i], b[j], t);
-            t           = p_fma(E2[j], b[i], t);
-            t           = p_fma(E3[i], D[j], t);
-            h[k]        = p_fma(E3[j], D[i], t);
-        }
-        const f2 tr  = p_add(p_add(gd[0], gd[1]), gd[2]);
-        const f2 nkd = p_mul(kw, p_mul(p_bc(-2.0f / 3.0f), tr));
-        const f2 k2  = p_add(kw, kw);
-        const f2 s00 = p_fma(k2, gd[0], nkd), s11 = p_fma(k2, gd[1], nkd), s22 = p_fma(k2, gd[2], nkd);
-        const f2 s01 = p_mul(kw, h[0]), s02 = p_mul(kw, h[1]), s12 = p_mul(kw, h[2]);
-        // sigma E for E = E1, E2, E3 (sigma symmetric)
-        auto sig = [&](const f2 (&E)[3], f2 (&o)[3]) {
-            o[0] = p_fma(s02, E[2], p_fma(s01, E[1], p_mul(s00, E[0])));
-            o[1] = p_fma(s12, E[2], p_fma(s11, E[1], p_mul(s01, E[0])));
-            o[2] = p_fma(s22, E[2], p_fma(s12, E[1], p_mul(s02, E[0])));
-        };
-        sig(E1, v1w[w]);
-        sig(E2, v2w[w]);
-        sig(E3, wvw[w]);
-    }
-    // corner 0: wedge 0 m=0; corner 3: wedge 1 m=0; corner 1: w0 m=1 + w1 m=2;
-    // corner 2: w0 m=2 + w1 m=1 (wedge_corner(1, m) = 3 - m)
-    const f2 m1 = make_float2(-1.0f, -1.0f);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const f2 v120 = p_add(v1w[0][c], v2w[0][c]);
-        const f2 v121 = p_add(v1w[1][c], v2w[1][c]);
-        const f2 rad  = p_add(wvw[0][c], wvw[1][c]);
-        const f2 lat1 = p_add(v1w[0][c], v2w[1][c]);
-        const f2 lat2 = p_add(v2w[0][c], v1w[1][c]);
-        out[0][0][c]  = p_mul(p_add(v120, wvw[0][c]), m1);
-        out[0][1][c]  = p_sub(wvw[0][c], v120);
-        out[3][0][c]  = p_mul(p_add(v121, wvw[1][c]), m1);
-        out[3][1][c]  = p_sub(wvw[1][c], v121);
-        out[1][0][c]  = p_sub(lat1, rad);
-        out[1][1][c]  = p_add(lat1, rad);
-        out[2][0][c]  = p_sub(lat2, rad);
-        out[2][1][c]  = p_add(lat2, rad);
-    }
-}
-
-// Packed FP32 pairs for the interior arithmetic: FP32, an even number of
-// radial cells per lane, apply mode (the diagonal mode stays scalar).
-template <typename T, int CPL, bool DIAG>
-inline constexpr bool kPackedPairs = std::is_same<T, float>::value && (CPL % 2 == 0) && !DIAG;
+constexpr int      kRing      = 6;  // staged rows
+constexpr uint32_t kSmemLimit = 227 * 1024;
 
 template <typename T>
 struct EddArgs {
-    int      nl, nr;
-    const T* coords;
-    const T* radii;
-    const T* k;    // nodal coefficient or nullptr
-    const T* kq0;  // per-cell coefficient or nullptr
-    const T* src[3];
-    T*       dst[3];
-    int      bc_cmb, bc_surf;
-    int      add;
-    int      ty, cx;
-    int*     err;
+    int         nl, nr;
+    const T*    geo;     // lateral table [10][nl - 1][nl][kGeo], entry y of a column x is strip y - 1
+    const T*    radii;
+    const T*    bdiag;   // [2 sides][10 nl nl][8]: diagonal (3), normal stiffness and normal (3) of the boundary nodes
+    const T*    k;       // nodal coefficient or nullptr
+    const T*    kq0;     // per-cell coefficient or nullptr
+    const T*    src[3];
+    T*          dst[3];
+    int         bc_cmb, bc_surf;
+    int         warps;       // compute warps
+    int         strips, ty;  // strips of a CTA (slots / nrc) and node lines it owns (<= strips - 1)
+    int         ytiles, rows, total_rows;
+    int*        err;
 };
 
 template <typename T>
-struct SmemLayout {
-    size_t   bar_off, ring_off, geo_off, nrm_off, bco_off, xch_off, total;
-    uint32_t rowcap;  // bytes per field per row buffer (16-aligned)
+struct EddSmem {
+    uint32_t bar, off, rec, edge, xch, ring, total;
+    uint32_t rowcap, slot, geo;  // bytes of one field of a staged row, of a ring slot and of its geometry
 };
 
-template <typename T, int CPL>
-__host__ __device__ inline SmemLayout<T> edd_smem_layout(int nr, int ty, int cx, int nfields)
+template <typename T>
+__host__ __device__ inline EddSmem<T> edd_smem(int nr, int warps, int strips)
 {
-    SmemLayout<T> L;
-    L.bar_off       = 0;  // 3 mbarriers, then the element offsets of the staged rows (3 slots x 4 fields, int)
-    L.rowcap        = static_cast<uint32_t>(((static_cast<size_t>(ty + 2) * nr * sizeof(T) + 16) + 15) / 16 * 16);
-    L.ring_off      = 128;
-    L.geo_off       = L.ring_off + static_cast<size_t>(3) * nfields * L.rowcap;
-    L.nrm_off       = L.geo_off + static_cast<size_t>(ty + 1) * (cx + 1) * 20 * sizeof(T);
-    L.bco_off       = L.nrm_off + static_cast<size_t>(ty + 1) * (cx + 1) * 12 * sizeof(T);
-    L.xch_off       = L.bco_off + static_cast<size_t>(ty + 1) * (cx + 1) * 36 * sizeof(T);
-    L.xch_off       = (L.xch_off + 15) / 16 * 16;
-    L.total         = L.xch_off + static_cast<size_t>(2) * (ty + 1) * 32 * 3 * (CPL + 1) * sizeof(T);
+    EddSmem<T>     L;
+    constexpr uint32_t t = sizeof(T);
+    const uint32_t     nw = static_cast<uint32_t>(warps), ns = static_cast<uint32_t>(strips);
+    L.bar    = 0;                                        // row landed, per ring slot
+    L.off    = 64;                                       // int4 per ring slot
+    L.rec    = L.off + kRing * 16;                       // [slot][column][side][4] T
+    L.edge   = L.rec + kRing * (ns + 1) * 8 * t;         // [parity][warp][6] T
+    L.xch    = (L.edge + 2 * nw * 6 * t + 15) / 16 * 16;  // [parity][warp][6][32] T
+    L.ring   = L.xch + 2 * nw * 6 * 32 * t;
+    L.rowcap = ((ns + 1) * static_cast<uint32_t>(nr) * t + 16 + 15) / 16 * 16;
+    L.geo    = ns * Shape<T>::kGeo * t;
+    L.slot   = L.geo + 4 * L.rowcap;                     // geometry, then 4 fields
+    L.total  = L.ring + kRing * L.slot;
     return L;
 }
 
-template <typename T, int CPL, bool DIAG>
-__global__ void __launch_bounds__(32 * MaxWarps<T>::value) epsdivdiv_kernel(EddArgs<T> A)
+// Position in the ring: slot and the parity of its current use.
+struct RingPos {
+    uint32_t slot = 0, parity = 0;
+    __device__ __forceinline__ void next()
+    {
+        if (++slot == kRing) {
+            slot = 0;
+            parity ^= 1u;
+        }
+    }
+};
+
+// One wedge: v1 = sigma g1, v2 = sigma g2, wv = sigma g3 for the lateral differences a, b, the scaled radial
+// difference D and the weight kw; g holds the wedge's nine table values.
+template <typename T>
+__device__ __forceinline__ void wedge_forces(const T (&g)[9], const T (&a)[3], const T (&b)[3], const T (&D)[3], T kw,
+                                             T (&v1)[3], T (&v2)[3], T (&wv)[3])
 {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int nl = A.nl, nr = A.nr;
-    const int ty = A.ty, cx = A.cx;
-    const int lane = threadIdx.x, w = threadIdx.y, nwarps = ty + 1;
-    const int d  = blockIdx.z;
-    const int y0 = blockIdx.x * ty;
-    const int xs = blockIdx.y * cx;
-    const int yc = y0 - 1 + w;  // cell strip of this warp
-    const bool q0 = A.kq0 != nullptr;
-    const int  nfields = q0 ? 3 : 4;
-
-    const SmemLayout<T> L   = edd_smem_layout<T, CPL>(nr, ty, cx, nfields);
-    uint64_t*           bar = reinterpret_cast<uint64_t*>(smem + L.bar_off);
-    int*                row_off = reinterpret_cast<int*>(smem + L.bar_off + 32);  // [slot][field]
-    unsigned char*      ring = smem + L.ring_off;
-    T*                  geo  = reinterpret_cast<T*>(smem + L.geo_off);
-    T*                  nrms = reinterpret_cast<T*>(smem + L.nrm_off);
-    T*                  bcof = reinterpret_cast<T*>(smem + L.bco_off);
-    T*                  xch  = reinterpret_cast<T*>(smem + L.xch_off);
-
-    const int ylo    = max(y0 - 1, 0);
-    const int yhi    = min(y0 + ty, nl - 1);
-    const int ncols  = yhi - ylo + 1;
-    const int nrows  = cx + 2;  // node rows xs-1 .. xs+cx
-    const int nsteps = cx + 1;  // cell columns xs-1 .. xs+cx-1
-    const T*  fields[4] = {A.src[0], A.src[1], A.src[2], A.k};
-
-    // The issuing thread records, per ring slot and field, the element offset (0..15 bytes / sizeof(T)) of the
-    // first staged element in the bulk-copied buffer (each field may sit at a different alignment); the
-    // mbarrier's release / acquire makes it visible with the row.
-    auto issue_row = [&](int i) {
-        const int xr   = xs - 1 + i;
-        const int slot = i % 3;
-        if (xr < 0 || xr >= nl) {
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(&bar[slot])) : "memory");
-            return;
-        }
-        const int64_t e0    = node_index(nl, nr, d, xr, ylo, 0);
-        uint32_t      total = 0;
-        uint32_t      bytes[4];
-        const T*      srcp[4];
-        for (int f = 0; f < nfields; ++f) {
-            const uint64_t a   = reinterpret_cast<uint64_t>(fields[f] + e0);
-            const uint64_t al  = a & ~uint64_t(15);
-            const uint32_t off = static_cast<uint32_t>(a - al);
-            bytes[f]           = (off + static_cast<uint32_t>(ncols) * nr * sizeof(T) + 15u) & ~15u;
-            srcp[f]            = reinterpret_cast<const T*>(al);
-            row_off[slot * 4 + f] = static_cast<int>(off / sizeof(T));
-            total += bytes[f];
-        }
-        mbar_arrive_expect_tx(&bar[slot], total);
-        for (int f = 0; f < nfields; ++f)
-            bulk_copy_g2s(ring + (static_cast<size_t>(slot) * nfields + f) * L.rowcap, srcp[f], bytes[f], &bar[slot]);
-    };
-
-    if (w == 0 && lane == 0) {
-        for (int s = 0; s < 3; ++s) mbar_init(&bar[s], 1);
-        fence_barrier_init();
+    T d[3], h[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) d[i] = fma(g[6 + i], D[i], fma(g[3 + i], b[i], g[i] * a[i]));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {  // pairs (0, 1), (0, 2), (1, 2)
+        const int i = k == 2 ? 1 : 0, j = k == 0 ? 1 : 2;
+        T         t = g[i] * a[j];
+        t           = fma(g[j], a[i], t);
+        t           = fma(g[3 + i], b[j], t);
+        t           = fma(g[3 + j], b[i], t);
+        t           = fma(g[6 + i], D[j], t);
+        h[k]        = fma(g[6 + j], D[i], t);
     }
-    __syncthreads();
-    int rows_issued = 0;  // meaningful on the issuing thread only
-    if (w == 0 && lane == 0) {
-        for (int i = 0; i < 3 && i < nrows; ++i) {
-            issue_row(i);
-            ++rows_issued;
-        }
-    }
-
-    // Lateral geometry (and corner normals) of this strip's cells for the
-    // chunk, one cell per lane.
-    const bool strip_ok = yc >= 0 && yc < nl - 1;
-    const bool has_fs   = (A.bc_cmb == 2) || (A.bc_surf == 2);
-    for (int i = lane; i < nsteps; i += 32) {
-        const int x  = xs - 1 + i;
-        T*        g  = geo + (static_cast<size_t>(w) * (cx + 1) + i) * 20;
-        T*        nv = nrms + (static_cast<size_t>(w) * (cx + 1) + i) * 12;
-        if (strip_ok && x >= 0 && x < nl - 1) {
-            column_geometry<T>(A.coords, nl, d, x, yc, g);
-            if (has_fs)
-                for (int q = 0; q < 4; ++q) {
-                    const T* c  = A.coords + node_index(nl, 1, d, x + (q & 1), yc + (q >> 1), 0) * 3;
-                    const T  in = T(1) / sqrt(c[0] * c[0] + c[1] * c[1] + c[2] * c[2]);
-                    for (int k = 0; k < 3; ++k) nv[q * 3 + k] = c[k] * in;
-                }
-            // boundary coefficients of the bottom (CMB) and top (surface) cells
-            for (int side = 0; side < 2; ++side) {
-                const int bc = side == 0 ? A.bc_cmb : A.bc_surf;
-                if (bc != 1 && bc != 2) continue;
-                const int rc = side == 0 ? 0 : nr - 2;
-                const T   r0 = A.radii[rc], r1 = A.radii[rc + 1];
-                const T   rm = T(0.5) * (r0 + r1), hdr = T(0.5) * (r1 - r0);
-                boundary_coefficients<T>(g, T(0.5) / rm, T(1) / (T(6) * hdr), rm * rm * hdr * (q0 ? T(1) : T(1) / T(6)),
-                                         side, bc, nv, bcof + ((static_cast<size_t>(w) * (cx + 1) + i) * 2 + side) * 18);
-            }
-        } else {
-            for (int v = 0; v < 20; ++v) g[v] = T(0);
-        }
-    }
-
-    // Per-lane radial constants.
-    T   alpha[CPL], beta[CPL], dfac[CPL];
-    int cbc[CPL][2];
+    const T k2 = kw + kw;
+    const T tr = (T(-1) / T(3)) * k2 * (d[0] + d[1] + d[2]);
+    const T s0 = fma(k2, d[0], tr), s1 = fma(k2, d[1], tr), s2 = fma(k2, d[2], tr);
+    const T s01 = kw * h[0], s02 = kw * h[1], s12 = kw * h[2];
 #pragma unroll
-    for (int j = 0; j < CPL; ++j) {
-        const int c = lane + 32 * j;
-        if (c < nr - 1) {
-            const T r0 = A.radii[c], r1 = A.radii[c + 1];
-            const T rm = T(0.5) * (r0 + r1), hdr = T(0.5) * (r1 - r0);
-            alpha[j]   = T(0.5) / rm;
-            beta[j]    = T(1) / (T(6) * hdr);
-            dfac[j]    = rm * rm * hdr * (q0 ? T(1) : T(1) / T(6));
-        } else {
-            alpha[j] = beta[j] = dfac[j] = T(0);
-        }
-        cbc[j][0] = (c == 0) ? A.bc_cmb : 0;
-        cbc[j][1] = (c == nr - 2) ? A.bc_surf : 0;
-    }
-    // Radial mapping: lane l holds cells l + 32 j (j < CPL), so shared-memory
-    // reads and global stores are consecutive across lanes. The top node nr-1
-    // is the extra node of the lane/iteration holding cell nr-2.
-    const int lane_top = (nr - 2) % 32;
-    const int j_top    = (nr - 2) / 32;
-
-    T xcarry[2][CPL + 1][3];
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int j = 0; j <= CPL; ++j)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) xcarry[a][j][c] = T(0);
-
-    __syncwarp();
-
-    bool ok        = true;
-    int  rows_done = 0;  // rows this thread has seen land, in order
-    for (int i = 0; i < nsteps; ++i) {
-        const int x = xs - 1 + i;
-        // rows i and i + 1 must be resident
-        if (ok && i == 0) {
-            ok = mbar_wait_bounded(&bar[0], 0);
-            rows_done += ok ? 1 : 0;
-        }
-        if (ok) {
-            ok = mbar_wait_bounded(&bar[(i + 1) % 3], ((i + 1) / 3) & 1);
-            rows_done += ok ? 1 : 0;
-        }
-        if (!ok) report_error(A.err, kDevMbarrierTimeout);
-        int offA[4], offB[4];
-#pragma unroll
-        for (int f = 0; f < 4; ++f) {
-            offA[f] = (f < nfields && x >= 0 && x < nl) ? row_off[(i % 3) * 4 + f] : 0;
-            offB[f] = (f < nfields && x + 1 >= 0 && x + 1 < nl) ? row_off[((i + 1) % 3) * 4 + f] : 0;
-        }
-        const T*  rowA = reinterpret_cast<const T*>(ring + static_cast<size_t>(i % 3) * nfields * L.rowcap);
-        const T*  rowB = reinterpret_cast<const T*>(ring + static_cast<size_t>((i + 1) % 3) * nfields * L.rowcap);
-        const bool cell_col_ok = strip_ok && x >= 0 && x < nl - 1;
-        const T*   g           = geo + (static_cast<size_t>(w) * (cx + 1) + i) * 20;
-
-        const T* nrm_col = nrms + (static_cast<size_t>(w) * (cx + 1) + i) * 12;
-
-        // Radial sums (node rc = bottom of cell rc + top of cell rc - 1) feed the
-        // x carry and the y exchange as soon as a node is complete.
-        T* slot_w = xch + (static_cast<size_t>(i & 1) * nwarps + w) * 3 * (CPL + 1) * 32 + lane;
-        T  keep[CPL + 1][3];
-        T  carry31[4][3];  // top of cell 32 j - 1 (lane 31, previous j)
-        auto finish_node = [&](int j, const T (&nv)[4][3]) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                keep[j][c]                = nv[0][c] + xcarry[0][j][c];
-                slot_w[(j * 3 + c) * 32] = nv[2][c] + xcarry[1][j][c];
-                xcarry[0][j][c]           = nv[1][c];
-                xcarry[1][j][c]           = nv[3][c];
-            }
-        };
-
-        // Staged inputs of cell rc of this column (the caller checks validity).
-        auto load_cell = [&](int rc, T (&u)[4][2][3], T (&ks)[4], T& kcell) {
-            const int e0 = (yc - ylo) * nr + rc;      // corners dy = 0
-            const int e1 = (yc + 1 - ylo) * nr + rc;  // corners dy = 1
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const unsigned char* row = reinterpret_cast<const unsigned char*>((q & 1) ? rowB : rowA);
-                const int*           off = (q & 1) ? offB : offA;
-                const int            e   = (q >> 1) ? e1 : e0;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const T* fr = reinterpret_cast<const T*>(row + static_cast<size_t>(c) * L.rowcap) + off[c];
-                    u[q][0][c]  = fr[e];
-                    u[q][1][c]  = fr[e + 1];
-                }
-                if (!q0) {
-                    const T* kr = reinterpret_cast<const T*>(row + static_cast<size_t>(3) * L.rowcap) + off[3];
-                    ks[q]       = kr[e] + kr[e + 1];
-                } else {
-                    ks[q] = T(0);
-                }
-            }
-            kcell = q0 ? A.kq0[node_index(nl - 1, nr - 1, d, x, yc, rc)] : T(0);
-        };
-        // Unmodified side-s values of cell rc (boundary rows).
-        auto load_raw = [&](int rc, int side, T (&raw)[4][3]) {
-            const int e0 = (yc - ylo) * nr + rc + side;
-            const int e1 = (yc + 1 - ylo) * nr + rc + side;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const unsigned char* row = reinterpret_cast<const unsigned char*>((q & 1) ? rowB : rowA);
-                const int*           off = (q & 1) ? offB : offA;
-                const int            e   = (q >> 1) ? e1 : e0;
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    raw[q][c] = reinterpret_cast<const T*>(row + static_cast<size_t>(c) * L.rowcap)[off[c] + e];
-            }
-        };
-        const T* bco_col = bcof + (static_cast<size_t>(w) * (cx + 1) + i) * 2 * 18;
-
-        // Scalar path: one cell (all modes).
-        auto scalar_cell = [&](int j, T (&out)[4][2][3]) {
-            const int rc = lane + 32 * j;
-            if (ok && cell_col_ok && rc < nr - 1) {
-                T u[4][2][3], ks[4], kcell;
-                load_cell(rc, u, ks, kcell);
-                if (DIAG) {
-                    const int bcs[2] = {cbc[j][0], cbc[j][1]};
-                    T         nrm[4][3];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            nrm[q][c] = has_fs ? nrm_col[q * 3 + c] : T(0);
-#pragma unroll
-                            for (int sd = 0; sd < 2; ++sd) out[q][sd][c] = T(0);
-                        }
-                    cell_apply<T, true>(u, ks, kcell, q0, g, alpha[j], beta[j], dfac[j], bcs, nrm, out);
-                } else {
-                    // boundary cells: only lane 0 (CMB, j = 0) and lane_top (surface, last j)
-                    const bool b0 = cbc[j][0] != 0;
-                    const bool b1 = cbc[j][1] != 0;
-                    T          un0[4], un1[4];
-                    if (b0) side_inputs<T>(u, 0, cbc[j][0], nrm_col, un0);
-                    if (b1) side_inputs<T>(u, 1, cbc[j][1], nrm_col, un1);
-                    hex_interior<T>(u, ks, kcell, q0, g, alpha[j], beta[j], dfac[j], out);
-#pragma unroll
-                    for (int side = 0; side < 2; ++side) {
-                        if (!(side == 0 ? b0 : b1)) continue;
-                        T raw[4][3];
-                        load_raw(rc, side, raw);
-                        side_outputs<T>(out, side, side == 0 ? cbc[j][0] : cbc[j][1], ks, kcell, q0,
-                                        bco_col + side * 18, nrm_col, raw, side == 0 ? un0 : un1);
-                    }
-                }
-            } else {
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int sd = 0; sd < 2; ++sd)
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) out[q][sd][c] = T(0);
-            }
-        };
-
-        // Radial sums of cell j's outputs into node values.
-        auto combine = [&](int j, const T (&out)[4][2][3]) {
-            T nv[4][3], top[4][3];
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    top[q][c]     = out[q][1][c];
-                    const T up    = shfl_up(top[q][c], 1);
-                    const T below = lane > 0 ? up : (j > 0 ? carry31[q][c] : T(0));
-                    nv[q][c]      = out[q][0][c] + below;
-                }
-            finish_node(j, nv);
-            if (j == j_top) finish_node(CPL, top);
-            if (j + 1 < CPL) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) carry31[q][c] = __shfl_sync(0xffffffffu, top[q][c], 31);
-            }
-        };
-
-        if constexpr (kPackedPairs<T, CPL, DIAG>) {
-            // FP32: cells (j, j + 1) of the lane as one packed pair
-#pragma unroll
-            for (int j = 0; j < CPL; j += 2) {
-                const int  rcA = lane + 32 * j, rcB = rcA + 32;
-                const bool vA  = ok && cell_col_ok && rcA < nr - 1;
-                const bool vB  = ok && cell_col_ok && rcB < nr - 1;
-                T          uA[4][2][3], uB[4][2][3], ksA[4], ksB[4], kA = T(0), kB = T(0);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    ksA[q] = ksB[q] = T(0);
-#pragma unroll
-                    for (int sd = 0; sd < 2; ++sd)
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) uA[q][sd][c] = uB[q][sd][c] = T(0);
-                }
-                if (vA) load_cell(rcA, uA, ksA, kA);
-                if (vB) load_cell(rcB, uB, ksB, kB);
-                // boundary cells: CMB is cell 0 (lane 0, j = 0), the surface cell nr - 2
-                const bool b0A = vA && cbc[j][0] != 0, b1A = vA && cbc[j][1] != 0;
-                const bool b0B = vB && cbc[j + 1][0] != 0, b1B = vB && cbc[j + 1][1] != 0;
-                T          un0A[4], un1A[4], un0B[4], un1B[4];
-                if (b0A) side_inputs<T>(uA, 0, cbc[j][0], nrm_col, un0A);
-                if (b1A) side_inputs<T>(uA, 1, cbc[j][1], nrm_col, un1A);
-                if (b0B) side_inputs<T>(uB, 0, cbc[j + 1][0], nrm_col, un0B);
-                if (b1B) side_inputs<T>(uB, 1, cbc[j + 1][1], nrm_col, un1B);
-                f2 u2[4][2][3], ks2[4], o2[4][2][3];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    ks2[q] = make_float2(ksA[q], ksB[q]);
-#pragma unroll
-                    for (int sd = 0; sd < 2; ++sd)
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) u2[q][sd][c] = make_float2(uA[q][sd][c], uB[q][sd][c]);
-                }
-                hex_interior_x2(u2, ks2, make_float2(kA, kB), q0, reinterpret_cast<const float*>(g),
-                                make_float2(alpha[j], alpha[j + 1]), make_float2(beta[j], beta[j + 1]),
-                                make_float2(dfac[j], dfac[j + 1]), o2);
-                T oA[4][2][3], oB[4][2][3];
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-#pragma unroll
-                    for (int sd = 0; sd < 2; ++sd)
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            oA[q][sd][c] = o2[q][sd][c].x;
-                            oB[q][sd][c] = o2[q][sd][c].y;
-                        }
-                if (b0A || b1A) {
-#pragma unroll
-                    for (int side = 0; side < 2; ++side) {
-                        if (!(side == 0 ? b0A : b1A)) continue;
-                        T raw[4][3];
-                        load_raw(rcA, side, raw);
-                        side_outputs<T>(oA, side, cbc[j][side], ksA, kA, q0, bco_col + side * 18, nrm_col, raw,
-                                        side == 0 ? un0A : un1A);
-                    }
-                }
-                if (b0B || b1B) {
-#pragma unroll
-                    for (int side = 0; side < 2; ++side) {
-                        if (!(side == 0 ? b0B : b1B)) continue;
-                        T raw[4][3];
-                        load_raw(rcB, side, raw);
-                        side_outputs<T>(oB, side, cbc[j + 1][side], ksB, kB, q0, bco_col + side * 18, nrm_col, raw,
-                                        side == 0 ? un0B : un1B);
-                    }
-                }
-                combine(j, oA);
-                combine(j + 1, oB);
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < CPL; ++j) {
-                T out[4][2][3];
-                scalar_cell(j, out);
-                combine(j, out);
-            }
-        }
-        __syncthreads();
-        if (w == 0 && lane == 0 && i + 3 < nrows) {
-            issue_row(i + 3);
-            ++rows_issued;
-        }
-
-        const int yn = yc;  // node line owned by warp w (w >= 1)
-        if (ok && w >= 1 && i >= 1 && x < nl && yn < nl) {
-            const T*  slot_p = xch + (static_cast<size_t>(i & 1) * nwarps + (w - 1)) * 3 * (CPL + 1) * 32 + lane;
-            const int obase  = ((d * nl + x) * nl + yn) * nr;  // 32-bit: the host limits a level to 2^31 nodes
-#pragma unroll
-            for (int j = 0; j <= CPL; ++j) {
-                const int rn = (j < CPL) ? lane + 32 * j : nr - 1;
-                const bool own = (j < CPL) ? (rn < nr - 1) : (lane == lane_top);
-                if (!own) continue;
-                const int id = obase + rn;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const T v = keep[j][c] + slot_p[(j * 3 + c) * 32];
-                    if (A.add)
-                        A.dst[c][id] += v;
-                    else
-                        A.dst[c][id] = v;
-                }
-            }
-        }
-    }
-    // After a timeout the issuing thread still waits (bounded) for every bulk
-    // copy it issued, so no copy lands in shared memory after the CTA retires.
-    if (w == 0 && lane == 0) {
-        for (int r = rows_done; r < rows_issued; ++r) (void)mbar_wait_bounded(&bar[r % 3], (r / 3) & 1, 100000000ull);
+    for (int m = 0; m < 3; ++m) {
+        T(&o)[3] = m == 0 ? v1 : (m == 1 ? v2 : wv);
+        const T x = g[3 * m], y = g[3 * m + 1], z = g[3 * m + 2];
+        o[0] = fma(s02, z, fma(s01, y, s0 * x));
+        o[1] = fma(s12, z, fma(s1, y, s01 * x));
+        o[2] = fma(s2, z, fma(s12, y, s02 * x));
     }
 }
 
-template <typename T, int CPL, bool DIAG>
-int launch_cfg(EddArgs<T> a, int nfields, cudaStream_t st)
+// MULTI: several strips share a warp (fewer than 32 radial cells); otherwise a strip takes nrc / 32 warps ("chunks").
+template <typename T, bool Q0, bool MULTI, bool ADD>
+__global__ void __launch_bounds__(Shape<T>::kThreads, 1) epsdivdiv_kernel(const __grid_constant__ EddArgs<T> A)
 {
-    constexpr size_t kSmemLimit = 227 * 1024;
-    SmemLayout<T>    L          = edd_smem_layout<T, CPL>(a.nr, a.ty, a.cx, nfields);
-    while (L.total > kSmemLimit && a.cx > 1) {
-        a.cx = (a.cx + 1) / 2;
-        L    = edd_smem_layout<T, CPL>(a.nr, a.ty, a.cx, nfields);
+    using Sh              = Shape<T>;
+    constexpr int kGeo    = Sh::kGeo;
+    constexpr int kMaxW   = Sh::kComputeWarps;
+    constexpr int kIssueWarp = kMaxW, kTreatWarp = kMaxW + 1;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int        nl = A.nl, nr = A.nr, nrc = nr - 1;
+    const int        lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int        strips = A.strips, ty = A.ty, ytiles = A.ytiles;
+    const EddSmem<T> L      = edd_smem<T>(nr, A.warps, strips);
+    uint64_t*        landed = reinterpret_cast<uint64_t*>(smem + L.bar);
+    int*             off    = reinterpret_cast<int*>(smem + L.off);
+    T*               rec    = reinterpret_cast<T*>(smem + L.rec);
+    const int        nchunks = MULTI ? 1 : nrc / 32;
+
+    // rows [R0, R1) of the flattened sequence (diamond, tile, x); staged: from one row before (unless the range
+    // starts a tile) to one row after (unless it ends one)
+    const int R0 = blockIdx.x * A.rows, R1 = min(R0 + A.rows, A.total_rows);
+    const int F0 = R0 - (R0 % nl != 0 ? 1 : 0);
+    const int F1 = R1 - 1 + ((R1 - 1) % nl < nl - 1 ? 1 : 0);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kRing; ++s) mbar_init(&landed[s], 1);
+        fence_barrier_init();
     }
-    if (L.total > kSmemLimit) return -5;
-    auto k = epsdivdiv_kernel<T, CPL, DIAG>;
+    // strips past the last cell column read their geometry from whatever the slot holds: start it at zero
+    for (uint32_t i = threadIdx.x; i < kRing * (L.geo / 4); i += Sh::kThreads) {
+        const uint32_t s = i / (L.geo / 4), e = i % (L.geo / 4);
+        *reinterpret_cast<uint32_t*>(smem + L.ring + s * L.slot + 4 * e) = 0u;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+
+    // One barrier a row for the compute warps and the two staging warps. Barrier B(f) ends the cells of row f: the
+    // exchange sums of row f are written, the reads of staged row f are done, row f + 2 has been treated.
+    const int  members     = 32 * (A.warps + 2);
+    const auto row_barrier = [&] { asm volatile("barrier.sync 1, %0;" ::"r"(members) : "memory"); };
+
+    if (w >= kMaxW) {
+        // ------------------------------------------------------------------
+        // Staging warps
+        // ------------------------------------------------------------------
+        if constexpr (Sh::kSplit) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Sh::kStageRegs));
+        if (w == kIssueWarp) {
+            const T* fields[4] = {A.src[0], A.src[1], A.src[2], A.k};
+            int      tile = F0 / nl, x = F0 - tile * nl, d = tile / ytiles, y0 = (tile - d * ytiles) * ty;
+            RingPos  pos;
+            bool     first_row = true;
+            auto     issue = [&] {
+                const int     ylo = max(y0 - 1, 0), ncols = min(y0 + strips - 1, nl - 1) - ylo + 1;
+                const int64_t e0  = node_index(nl, nr, d, x, ylo, 0);
+                // field i into the slot: 16-byte aligned copy around n elements from p; returns the bytes
+                const uint32_t first = L.ring + pos.slot * L.slot + L.geo;
+                uint32_t       total = 0;
+                auto bytes_of = [&](const T* p, int n) {
+                    return ((static_cast<uint32_t>(reinterpret_cast<uint64_t>(p)) & 15u) + static_cast<uint32_t>(n * static_cast<int>(sizeof(T))) + 15u) & ~15u;
+                };
+                // the cell column behind this row: geometry of its strips, and their coefficients (Q0)
+                const bool column = x > 0 && !first_row;
+                const T*   q0p    = nullptr;
+                int        nq     = 0;
+                if (Q0 && column) {
+                    q0p = A.kq0 + node_index(nl - 1, nrc, d, x - 1, ylo, 0);
+                    nq  = (min(y0 + strips - 2, nl - 2) - ylo + 1) * nrc;
+                }
+                const int ngeo = column ? min(strips, nl - y0) : 0;  // entries y0 .. (entry y is strip y - 1)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const T* p = Q0 && i == 3 ? q0p : fields[i] + e0;
+                    const int n = Q0 && i == 3 ? nq : ncols * nr;
+                    if (n > 0) total += bytes_of(p, n);
+                    off[4 * pos.slot + i] = static_cast<int>(first + i * L.rowcap + (static_cast<uint32_t>(reinterpret_cast<uint64_t>(p)) & 15u));
+                }
+                total += static_cast<uint32_t>(ngeo * kGeo * static_cast<int>(sizeof(T)));
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                mbar_arrive_expect_tx(&landed[pos.slot], total);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const T* p = Q0 && i == 3 ? q0p : fields[i] + e0;
+                    const int n = Q0 && i == 3 ? nq : ncols * nr;
+                    if (n > 0)
+                        bulk_copy_g2s(smem + first + i * L.rowcap,
+                                      reinterpret_cast<const void*>(reinterpret_cast<uint64_t>(p) & ~uint64_t(15)),
+                                      bytes_of(p, n), &landed[pos.slot]);
+                }
+                if (ngeo > 0)
+                    bulk_copy_g2s(smem + first - L.geo,
+                                  A.geo + ((static_cast<int64_t>(d) * (nl - 1) + (x - 1)) * nl + y0) * kGeo,
+                                  static_cast<uint32_t>(ngeo * kGeo * static_cast<int>(sizeof(T))), &landed[pos.slot]);
+                first_row = false;
+                pos.next();
+                if (++x == nl) {
+                    x = 0;
+                    if (++tile % ytiles == 0) {
+                        ++d;
+                        y0 = 0;
+                    } else {
+                        y0 += ty;
+                    }
+                }
+            };
+            int next = F0;
+            if (lane == 0)
+                for (int i = 0; i < kRing && next <= F1; ++i, ++next) issue();
+            row_barrier();
+            for (int f = F0; f < R1; ++f) {
+                // the slot of row f - 1 is free: its last readers have passed B(f - 1)
+                if (lane == 0 && f > F0 && next <= F1) {
+                    issue();
+                    ++next;
+                }
+                row_barrier();
+            }
+            return;
+        }
+        if (w != kTreatWarp) return;
+        // Rows in order: wait for the copies and apply the input side of the boundary treatment to the two boundary
+        // planes (Dirichlet: input 0, record diag u; free slip: tangential part, record (n, Ann n.u)).
+        const bool any_bc = A.bc_cmb != 0 || A.bc_surf != 0;
+        int        tile = F0 / nl, x = F0 - tile * nl, d = tile / ytiles, y0 = (tile - d * ytiles) * ty;
+        RingPos    pos;
+        bool       ok = true;
+        auto       treat = [&] {
+            const int ylo = max(y0 - 1, 0), ncols = min(y0 + strips - 1, nl - 1) - ylo + 1;
+            bool      waited = false;
+            for (int i = lane; i - lane < (any_bc ? 2 * ncols : 1); i += 32) {
+                const bool on   = any_bc && i < 2 * ncols;
+                const int  col  = on ? i >> 1 : 0, side = i & 1;
+                const int  bc   = side == 0 ? A.bc_cmb : A.bc_surf;
+                T          t[8] = {};  // diagonal, normal stiffness, normal
+                if (on && bc != 0) {
+                    const T* p = A.bdiag + (static_cast<int64_t>(side) * 10 * nl * nl + lat_index3(nl, d, x, ylo + col)) * 8;
+#pragma unroll
+                    for (int q = 0; q < 7; ++q) t[q] = p[q];
+                }
+                if (!waited) {
+                    waited = true;
+                    if (ok) ok = mbar_wait_bounded(&landed[pos.slot], pos.parity);
+                    if (!ok) report_error(A.err, kDevMbarrierTimeout);
+                }
+                if (!on || bc == 0) continue;
+                T* u[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    u[c] = reinterpret_cast<T*>(smem + off[4 * pos.slot + c]) + col * nr + (side == 0 ? 0 : nrc);
+                const T u0 = *u[0], u1 = *u[1], u2 = *u[2];
+                T*      o  = rec + (pos.slot * static_cast<uint32_t>(strips + 1) + (ylo - (y0 - 1)) + col) * 8 + side * 4;
+                if (bc == 1) {
+                    o[0] = t[0] * u0, o[1] = t[1] * u1, o[2] = t[2] * u2;
+                    *u[0] = T(0), *u[1] = T(0), *u[2] = T(0);
+                } else {
+                    const T un = t[4] * u0 + t[5] * u1 + t[6] * u2;
+                    o[0] = t[4], o[1] = t[5], o[2] = t[6], o[3] = t[3] * un;
+                    *u[0] = u0 - un * t[4], *u[1] = u1 - un * t[5], *u[2] = u2 - un * t[6];
+                }
+            }
+            // these writes precede the slot's next copy
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            pos.next();
+            if (++x == nl) {
+                x = 0;
+                if (++tile % ytiles == 0) {
+                    ++d;
+                    y0 = 0;
+                } else {
+                    y0 += ty;
+                }
+            }
+        };
+        treat();
+        if (F1 > F0) treat();
+        row_barrier();
+        for (int f = F0; f < R1; ++f) {
+            if (f + 2 <= F1) treat();
+            row_barrier();
+        }
+        // every copy has landed: all rows were waited for above, or, after a timeout, here
+        if (!ok)
+            for (int s = 0; s < kRing; ++s) (void)mbar_wait_bounded(&landed[s], 0, 100000000ull);
+        return;
+    }
+
+    if constexpr (Sh::kSplit) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Sh::kComputeRegs));
+    if (w >= A.warps) return;
+    // ----------------------------------------------------------------------
+    // Compute warps: one cell per lane.
+    // ----------------------------------------------------------------------
+    T*         xch   = reinterpret_cast<T*>(smem + L.xch);
+    T*         edge  = reinterpret_cast<T*>(smem + L.edge);
+    const int  chunk = MULTI ? 0 : w % nchunks;
+    const int  spw   = MULTI ? 32 / nrc : 1;
+    const int  strip = MULTI ? w * spw + lane / nrc : w / nchunks;
+    const int  rc    = MULTI ? lane % nrc : chunk * 32 + lane;
+    const int  below = MULTI ? max(strip - 1, 0) : 0;
+    // (strip - 1, rc) in the exchange buffer of one parity; the lane whose top is below this lane's cell
+    const int  prev       = MULTI ? (below / spw) * 6 * 32 + (below % spw) * nrc + rc : max(w - nchunks, 0) * 6 * 32 + lane;
+    const int  below_lane = MULTI ? (lane & ~(nrc - 1)) | ((lane + nrc - 1) & (nrc - 1)) : (lane + 31) & 31;
+    const bool last_chunk = chunk + 1 == nchunks;
+    const bool first_node = rc == 0, last_node = rc == nrc - 1;  // this lane holds the strip's node 0 / nr - 1
+
+    // radial constants: rho = beta / alpha = 2 r_mid / (3 dr), weight dr / 8 (/ 6 for the nodal mean)
+    auto rho_of = [&](int c) { return (A.radii[c] + A.radii[c + 1]) / (T(3) * (A.radii[c + 1] - A.radii[c])); };
+    const T rho = rho_of(rc);
+    const T wr  = (A.radii[rc + 1] - A.radii[rc]) / (Q0 ? T(8) : T(48));
+
+    const T rho_low = !MULTI && chunk > 0 ? rho_of(rc - 1) : T(0);  // of the cell below the chunk
+
+    // a node column of the sweep: corner sums / differences / coefficients of nodes y (0) and y + 1 (1)
+    struct Column {
+        T S[2][3], D[2][3], k[2];
+    } o = {};
+    // forces the column's cells left on it (lateral part of node y + 1 with opposite sign)
+    T         cL[2][3], cR[2][3];
+    T         kL[3], kR[3];  // this warp's sums of node (x, y)
+    int       x = 0;
+    int       e0 = 0, q0 = 0;  // byte offsets of the cell's bottom node y (and cell coefficient) in a staged field
+    int       id = 0;          // node (x, y, rc)
+    bool      valid = false, own = false, some = true, any_own = true;
+    const int pitch = nr * static_cast<int>(sizeof(T));
+    uint32_t  slot = 0, par = 0;  // ring slot of row f, exchange parity of the step
+    const uint32_t half = A.warps * (6 * 32);
+    T* const       out  = xch + w * (6 * 32) + lane;
+    const T* const in   = xch + prev;
+
+    auto put = [&](int c, int i, T v) {
+        T* p = A.dst[c] + i;
+        if (ADD) v += *p;
+        *p = v;
+    };
+    auto load_column = [&](uint32_t rslot, Column& C) {
+        const int4 o4    = *reinterpret_cast<const int4*>(off + 4 * rslot);
+        const int  at[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+        for (int fld = 0; fld < (Q0 ? 3 : 4); ++fld) {
+            const unsigned char* p0 = smem + at[fld] + e0;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const T* p   = reinterpret_cast<const T*>(p0 + q * pitch);
+                T        bot = p[0], top = p[1];
+                if (MULTI && !valid) bot = top = T(0);
+                if (fld < 3) {
+                    C.S[q][fld] = top + bot;
+                    C.D[q][fld] = top - bot;
+                } else {
+                    C.k[q] = wr * (top + bot);
+                }
+            }
+        }
+    };
+    // Cells between rows f and f + 1 (slot n1): sums of row f into kL / kR and the exchange, of row f + 1 into cL / cR.
+    auto cells = [&](uint32_t n1) {
+        Column n;
+        load_column(n1, n);
+        T kw0, kw1;
+        if constexpr (Q0) {
+            T kc = *reinterpret_cast<const T*>(smem + off[4 * n1 + 3] + q0);
+            if (MULTI && !valid) kc = T(0);
+            kw0 = kw1 = wr * kc;
+        } else {
+            const T k12 = n.k[0] + o.k[1];
+            kw0         = o.k[0] + k12;
+            kw1         = n.k[1] + k12;
+        }
+        // corners: 0 = (x, y) old 0, 2 = (x, y + 1) old 1, 1 = (x + 1, y) new 0, 3 = (x + 1, y + 1) new 1;
+        // wedge 0 has nodes 0, 1, 2, wedge 1 has nodes 3, 2, 1
+        T a[3], b[3], D[3], m[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            a[c] = n.S[0][c] - o.S[0][c];
+            b[c] = o.S[1][c] - o.S[0][c];
+            m[c] = rho * (n.D[0][c] + o.D[1][c]);
+            D[c] = fma(rho, o.D[0][c], m[c]);
+        }
+        const T* gp = reinterpret_cast<const T*>(smem + L.ring + n1 * L.slot) + strip * kGeo;
+        auto     load_geo = [&](int w2, T (&g)[9]) {
+            const T* q = gp + w2 * (kGeo / 2);
+            if constexpr (sizeof(T) == 8) {
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) {
+                    const double2 t = *reinterpret_cast<const double2*>(q + i);
+                    g[i] = t.x, g[i + 1] = t.y;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; i += 4) {
+                    const float4 t = *reinterpret_cast<const float4*>(q + i);
+                    g[i] = t.x, g[i + 1] = t.y, g[i + 2] = t.z, g[i + 3] = t.w;
+                }
+            }
+            g[8] = q[8];
+        };
+        T g[9], v1[3], v2[3], wv[3], r0[3], sL[3];
+        load_geo(0, g);
+        wedge_forces(g, a, b, D, kw0, v1, v2, wv);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            kL[c]    = cL[0][c] - (v1[c] + v2[c]);
+            kR[c]    = cR[0][c] + wv[c];
+            sL[c]    = v2[c] - cL[1][c];
+            cL[0][c] = v1[c];
+            r0[c]    = wv[c];
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            a[c] = o.S[1][c] - n.S[1][c];
+            b[c] = n.S[0][c] - n.S[1][c];
+            D[c] = fma(rho, n.D[1][c], m[c]);
+        }
+        load_geo(1, g);
+        wedge_forces(g, a, b, D, kw1, v1, v2, wv);
+        T* so = out + par;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const T rad      = r0[c] + wv[c];
+            so[c * 32]       = sL[c] + v1[c];
+            so[(3 + c) * 32] = cR[1][c] + rad;
+            cL[0][c] += v2[c];
+            cR[0][c] = rad;
+            cL[1][c] = v1[c] + v2[c];
+            cR[1][c] = wv[c];
+        }
+        o = n;
+    };
+    // no cells beyond row f: what the column before left
+    auto no_cells = [&] {
+        T* so = out + par;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            kL[c]            = cL[0][c];
+            kR[c]            = cR[0][c];
+            so[c * 32]       = -cL[1][c];
+            so[(3 + c) * 32] = cR[1][c];
+        }
+    };
+    // Node values of row f: own sums plus those of the strip below in y.
+    auto nodes = [&](bool write) {
+        if (!MULTI && !last_chunk && lane == 31) {  // own sums of the chunk's last cell for the chunk above
+            T* q = edge + (par == 0 ? 0 : A.warps * 6) + w * 6;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                q[c]     = kL[c];
+                q[3 + c] = kR[c];
+            }
+        }
+        row_barrier();
+        if (write && any_own) {
+            const T* ps = in + par;
+            T        bot[3], top[3], low[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const T l = kL[c] + ps[c * 32], r = kR[c] + ps[(3 + c) * 32];
+                bot[c] = fma(-rho, r, l);
+                top[c] = fma(rho, r, l);
+                low[c] = __shfl_sync(0xffffffffu, top[c], below_lane);
+                if (MULTI ? first_node : lane == 0) low[c] = T(0);
+            }
+            if (!MULTI && chunk > 0 && lane == 0) {  // the cell below belongs to the warp before
+                const T* q  = edge + (par == 0 ? 0 : A.warps * 6) + (w - 1) * 6;
+                const T* q2 = ps - 6 * 32 + 31;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) low[c] = fma(rho_low, q[3 + c] + q2[(3 + c) * 32], q[c] + q2[c * 32]);
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) bot[c] += low[c];
+            if (!MULTI || own) {
+                if (first_node || last_node) {  // nrc >= 2: never both
+                    const int bc = first_node ? A.bc_cmb : A.bc_surf;
+                    const T*  q  = rec + (slot * static_cast<uint32_t>(strips + 1) + strip) * 8 + (first_node ? 0 : 4);
+                    T         v[3];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) v[c] = first_node ? bot[c] : top[c];
+                    if (bc == 1) {
+                        v[0] = q[0], v[1] = q[1], v[2] = q[2];
+                    } else if (bc == 2) {
+                        const T cr = q[3] - (q[0] * v[0] + q[1] * v[1] + q[2] * v[2]);
+                        v[0] += cr * q[0], v[1] += cr * q[1], v[2] += cr * q[2];
+                    }
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        if (first_node)
+                            bot[c] = v[c];
+                        else
+                            put(c, id + 1, v[c]);
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 3; ++c) put(c, id, bot[c]);
+            }
+        }
+        par = half - par;
+        id += nl * nr;
+    };
+
+    row_barrier();
+    for (int f = F0; f < R1;) {
+        // rows of one tile: x .. xe - 1
+        const int tile = f / nl, d = tile / ytiles, y0 = (tile - d * ytiles) * ty;
+        x            = f - tile * nl;
+        const int xe = min(nl, x + R1 - f), yc = y0 - 1 + strip, col0 = max(strip - (y0 == 0 ? 1 : 0), 0);
+        valid   = yc >= 0 && yc < nl - 1;
+        own     = strip >= 1 && strip <= ty && yc < nl;
+        e0      = (col0 * nr + rc) * static_cast<int>(sizeof(T));
+        q0      = (col0 * nrc + rc) * static_cast<int>(sizeof(T));
+        id      = ((d * nl + x) * nl + yc) * nr + rc;  // 32-bit: the host limits a level to 2^31 nodes
+        some    = MULTI ? __any_sync(0xffffffffu, valid) : valid;
+        any_own = MULTI ? __any_sync(0xffffffffu, own) : own;
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) cL[q][c] = cR[q][c] = T(0);
+        if (some && x < nl - 1) load_column(slot, o);
+        const int cols = min(xe, nl - 1);
+        // FP64 has registers for two columns a trip, which saves copying the column behind (105 -> 102 us at level 6);
+        // FP32 spills with it (69 -> 73 us)
+#pragma unroll(sizeof(T) == 8 ? 2 : 1)
+        for (; x < cols; ++x, ++f) {
+            const uint32_t n1 = slot + 1 == kRing ? 0 : slot + 1;
+            if (some)
+                cells(n1);
+            else
+                no_cells();
+            nodes(f >= R0);
+            slot = n1;
+        }
+        if (x < xe) {  // the tile's last row
+            no_cells();
+            nodes(f >= R0);
+            slot = slot + 1 == kRing ? 0 : slot + 1;
+            ++f;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Diagonal. f(g, kw) for every wedge around node (d, x, y, r) of this diamond: physical gradient g of the node's
+// shape function and weight kw = k |det J|.
+// ---------------------------------------------------------------------------
+template <typename G, typename K, typename F>
+__device__ __forceinline__ void node_wedges(int nl, int nr, const G* colgeo, const G* radgeo, const K* k, const K* kq0,
+                                            int d, int x, int y, int r, F&& f)
+{
+    for (int ab = 0; ab < 4; ++ab) {
+        const int xc = x - (ab & 1), yc = y - (ab >> 1);
+        if (xc < 0 || yc < 0 || xc > nl - 2 || yc > nl - 2) continue;
+        const int col = (d * (nl - 1) + xc) * (nl - 1) + yc;
+        for (int top = 0; top < 2; ++top) {
+            const int rc = r - top;
+            if (rc < 0 || rc > nr - 2) continue;
+            const G alpha = radgeo[3 * rc], beta = radgeo[3 * rc + 1], dfac = radgeo[3 * rc + 2];
+            for (int w = 0; w < 2; ++w) {
+                const int m = w == 0 ? ab : 3 - ab;  // lateral index of corner ab in wedge w
+                if (m > 2) continue;
+                G kv;
+                if (kq0) {
+                    kv = static_cast<G>(kq0[static_cast<int64_t>(col) * (nr - 1) + rc]);
+                } else {
+                    kv = G(0);
+                    for (int j = 0; j < 3; ++j) {
+                        const int     q  = wedge_corner(w, j);
+                        const int64_t id = node_index(nl, nr, d, xc + (q & 1), yc + (q >> 1), rc);
+                        kv += static_cast<G>(k[id]) + static_cast<G>(k[id + 1]);
+                    }
+                    kv *= G(1) / G(6);
+                }
+                const G* gw = colgeo + static_cast<int64_t>(col) * 20 + 10 * w;
+                G        g[3];
+                for (int i = 0; i < 3; ++i) {
+                    const G lat = m == 0 ? -(gw[i] + gw[3 + i]) : (m == 1 ? gw[i] : gw[3 + i]);
+                    g[i]        = alpha * lat + (top ? beta : -beta) * gw[6 + i];
+                }
+                f(g, kv * gw[9] * dfac);
+            }
+        }
+    }
+}
+
+// Diagonal mode: dst = diag(A) src, one thread per node; on free-slip nodes the diagonal in the node's
+// normal-tangential frame.
+template <typename T>
+__global__ void __launch_bounds__(256) edd_diagonal_kernel(EddLaunch<T> A, int n, Decoder rad, Decoder lat)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    int d, x, y, r, col;
+    decode4(i, rad, lat, d, x, y, r, col);
+    const int bc   = r == 0 ? A.bc_cmb : (r == A.nr - 1 ? A.bc_surf : 0);
+    const T   u[3] = {A.src[0][i], A.src[1][i], A.src[2][i]};
+    T         o[3];
+    T         R[3][3] = {};
+    if (bc == 2) {
+        const T* c  = A.coords + static_cast<int64_t>(col) * 3;
+        const T  in = T(1) / sqrt(c[0] * c[0] + c[1] * c[1] + c[2] * c[2]);
+        const T  nv[3] = {c[0] * in, c[1] * in, c[2] * in};
+        trafo_nt(nv, R);
+    }
+    T dg[3] = {T(0), T(0), T(0)};
+    node_wedges(A.nl, A.nr, A.colgeo, A.radgeo, A.k, A.kq0, d, x, y, r, [&](const T(&g)[3], T kw) {
+        const T gg = g[0] * g[0] + g[1] * g[1] + g[2] * g[2];
+        for (int c = 0; c < 3; ++c) {
+            const T q = bc == 2 ? R[c][0] * g[0] + R[c][1] * g[1] + R[c][2] * g[2] : g[c];
+            dg[c] += kw * (gg + q * q * (T(1) / T(3)));
+        }
+    });
+    if (bc == 2) {
+        T v[3];
+        for (int a = 0; a < 3; ++a) v[a] = dg[a] * (R[a][0] * u[0] + R[a][1] * u[1] + R[a][2] * u[2]);
+        for (int c = 0; c < 3; ++c) o[c] = R[0][c] * v[0] + R[1][c] * v[1] + R[2][c] * v[2];
+    } else {
+        for (int c = 0; c < 3; ++c) o[c] = dg[c] * u[c];
+    }
+    for (int c = 0; c < 3; ++c) A.dst[c][i] = A.add ? A.dst[c][i] + o[c] : o[c];
+}
+
+// Boundary rows: for each node of the two boundary planes the diagonal (3 values) and the normal stiffness
+// sum kw (|g|^2 + (n.g)^2 / 3), of this diamond's cells, and the unit normal. Independent of the boundary conditions.
+template <typename T>
+__global__ void __launch_bounds__(256) edd_boundary_kernel(int nl, int nr, const double* coords, const double* colgeo,
+                                                           const double* radgeo, const T* k, const T* kq0, T* out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, n = 10 * nl * nl;
+    if (i >= 2 * n) return;
+    const int    side = i / n, c = i % n;
+    const int    y = c % nl, x = (c / nl) % nl, d = c / (nl * nl);
+    const double p0 = coords[3 * c], p1 = coords[3 * c + 1], p2 = coords[3 * c + 2];
+    const double in = 1.0 / sqrt(p0 * p0 + p1 * p1 + p2 * p2);
+    double       dg[3] = {0.0, 0.0, 0.0}, ann = 0.0;
+    node_wedges(nl, nr, colgeo, radgeo, k, kq0, d, x, y, side == 0 ? 0 : nr - 1, [&](const double(&g)[3], double kw) {
+        const double gg = g[0] * g[0] + g[1] * g[1] + g[2] * g[2];
+        for (int q = 0; q < 3; ++q) dg[q] += kw * (gg + g[q] * g[q] * (1.0 / 3.0));
+        const double ng = (p0 * g[0] + p1 * g[1] + p2 * g[2]) * in;
+        ann += kw * (gg + ng * ng * (1.0 / 3.0));
+    });
+    T* o = out + static_cast<int64_t>(i) * 8;
+    for (int q = 0; q < 3; ++q) o[q] = static_cast<T>(dg[q]);
+    o[3] = static_cast<T>(ann);
+    o[4] = static_cast<T>(p0 * in), o[5] = static_cast<T>(p1 * in), o[6] = static_cast<T>(p2 * in), o[7] = T(0);
+}
+
+// Double-double arithmetic for the lateral table (Dekker, Numer. Math. 18, 1971; products by fused multiply-add), so
+// that its entries are the rounded exact values: they enter the apply twice, on the input and on the output side.
+struct Dd {
+    double h, l;
+};
+__device__ __forceinline__ Dd dd_norm(double a, double b)
+{
+    const double s = a + b;
+    return {s, b - (s - a)};
+}
+__device__ __forceinline__ Dd dd_add(Dd a, Dd b)
+{
+    const double s = a.h + b.h, v = s - a.h;
+    return dd_norm(s, ((a.h - (s - v)) + (b.h - v)) + (a.l + b.l));
+}
+__device__ __forceinline__ Dd dd_neg(Dd a) { return {-a.h, -a.l}; }
+__device__ __forceinline__ Dd dd_mul(Dd a, Dd b)
+{
+    const double p = a.h * b.h;
+    return dd_norm(p, fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
+}
+__device__ __forceinline__ Dd dd_div(Dd a, Dd b)
+{
+    const double q = a.h / b.h;
+    const Dd     r = dd_add(a, dd_neg(dd_mul(b, {q, 0.0})));
+    return dd_norm(q, (r.h + r.l) / b.h);
+}
+__device__ __forceinline__ Dd dd_sqrt(Dd a)
+{
+    const double q = sqrt(a.h);
+    const Dd     r = dd_add(a, dd_neg(dd_mul({q, 0.0}, {q, 0.0})));
+    return dd_norm(q, (r.h + r.l) / (2.0 * q));
+}
+
+// Lateral table: entry (d, x, e) holds sqrt|det M| (e1, e2, e3) of both wedges of column y = e - 1 (zeros off the mesh).
+// e1 = a2 x a3 / det and so on, so sqrt|det M| e1 = a2 x a3 / (sign(det) sqrt|det M|).
+template <typename T>
+__global__ void __launch_bounds__(128) edd_lateral_kernel(int nl, const double* coords, T* out)
+{
+    constexpr int kGeo = Shape<T>::kGeo;
+    const int     i    = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 10 * (nl - 1) * nl) return;
+    const int e = i % nl, x = (i / nl) % (nl - 1), d = i / (nl * (nl - 1));
+    T*        o = out + static_cast<int64_t>(i) * kGeo;
+    for (int v = 0; v < kGeo; ++v) o[v] = T(0);
+    if (e == 0) return;
+    for (int w = 0; w < 2; ++w) {
+        Dd a[3][3];
+        for (int c = 0; c < 3; ++c) {
+            Dd p[3];
+            for (int m = 0; m < 3; ++m) {
+                const int q = wedge_corner(w, m);
+                p[m]        = {coords[lat_index3(nl, d, x + (q & 1), e - 1 + (q >> 1)) * 3 + c], 0.0};
+            }
+            a[0][c] = dd_add(p[1], dd_neg(p[0]));
+            a[1][c] = dd_add(p[2], dd_neg(p[0]));
+            a[2][c] = dd_div(dd_add(dd_add(p[0], p[1]), p[2]), {3.0, 0.0});
+        }
+        Dd n[3][3], det = {0.0, 0.0};
+        for (int k = 0; k < 3; ++k)
+            for (int c = 0; c < 3; ++c) {
+                const Dd *u = a[(k + 1) % 3], *v = a[(k + 2) % 3];
+                n[k][c] = dd_add(dd_mul(u[(c + 1) % 3], v[(c + 2) % 3]), dd_neg(dd_mul(u[(c + 2) % 3], v[(c + 1) % 3])));
+            }
+        for (int c = 0; c < 3; ++c) det = dd_add(det, dd_mul(a[0][c], n[0][c]));
+        const Dd s = det.h < 0.0 ? dd_neg(dd_sqrt(dd_neg(det))) : dd_sqrt(det);
+        for (int k = 0; k < 3; ++k)
+            for (int c = 0; c < 3; ++c) o[w * (kGeo / 2) + 3 * k + c] = static_cast<T>(dd_div(n[k][c], s).h);
+    }
+}
+
+template <typename T, bool Q0, bool MULTI, bool ADD>
+int launch_cfg(const EddArgs<T>& a, size_t smem, int ctas, cudaStream_t st)
+{
+    auto k = epsdivdiv_kernel<T, Q0, MULTI, ADD>;
     // the dynamic shared-memory limit is a per-device attribute of the kernel:
     // raise it once per device, only upwards; the check, the attribute call
     // and the record happen under one lock so racing threads cannot lower it
@@ -613,84 +797,159 @@ int launch_cfg(EddArgs<T> a, int nfields, cudaStream_t st)
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -1;
     {
         std::lock_guard<std::mutex> lock(mu);
-        if (L.total > configured[dev]) {
-            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(L.total)) !=
+        if (smem > configured[dev]) {
+            // the compute warps wait for registers that the block must hold from its launch
+            cudaFuncAttributes at;
+            if (cudaFuncGetAttributes(&at, k) != cudaSuccess || (Shape<T>::kSplit && at.numRegs * 4 < 3 * Shape<T>::kComputeRegs + Shape<T>::kStageRegs))
+                return -7;
+            if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
                 cudaSuccess)
                 return -1;
-            configured[dev] = L.total;
+            configured[dev] = smem;
         }
     }
-    const int nl = a.nl;
-    dim3      grid((nl + a.ty - 1) / a.ty, (nl + a.cx - 1) / a.cx, 10);
-    dim3      block(32, a.ty + 1);
-    k<<<grid, block, L.total, st>>>(a);
+    k<<<ctas, Shape<T>::kThreads, smem, st>>>(a);
     note_launch();
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-template <typename T>
-int launch(const EddArgs<T>& a, bool diag, cudaStream_t st)
+int sm_count()
 {
-    const int cells = a.nr - 1;
-    const int nf    = a.kq0 ? 3 : 4;
-    if (cells <= 32) return diag ? launch_cfg<T, 1, true>(a, nf, st) : launch_cfg<T, 1, false>(a, nf, st);
-    if (cells <= 64) return diag ? launch_cfg<T, 2, true>(a, nf, st) : launch_cfg<T, 2, false>(a, nf, st);
-    if (cells <= 128) return diag ? launch_cfg<T, 4, true>(a, nf, st) : launch_cfg<T, 4, false>(a, nf, st);
-    return -3;
+    static std::atomic<int> counts[kMaxDevices];
+    int                     dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -1;
+    int sms = counts[dev].load(std::memory_order_relaxed);
+    if (sms == 0) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+        counts[dev].store(sms, std::memory_order_relaxed);
+    }
+    return sms;
 }
 
 }  // namespace
 
 template <typename T>
+EddPlan edd_plan(int nl, int nr, int sms, int tile_y, int chunk_x)
+{
+    // Warps come in whole strips. The cost of a shape is rows per CTA (plus the repeated column) times the time of a
+    // row: the issue time of its warps, four schedulers at a time, plus a latency floor of about five warps. It picks
+    // 12 strips at level 6 in FP32 (69 us; 11 strips 80 us) and 6 in FP64 (105 us; 4 strips 140 us).
+    const int nrc = nr - 1, slots = 32;
+    const int wps = nrc > slots ? nrc / slots : 1;  // warps per strip
+    const int spw = nrc < slots ? slots / nrc : 1;  // strips per warp
+    EddPlan   best;
+    double    cost = -1.0;
+    for (int w = wps; w <= Shape<T>::kComputeWarps; w += wps) {
+        const int strips = w / wps * spw;
+        if (strips < 2) continue;
+        if (edd_smem<T>(nr, w, strips).total > kSmemLimit) break;
+        EddPlan p;
+        p.warps  = w;
+        p.strips = strips;
+        p.ty     = std::min(strips - 1, nl);
+        if (tile_y > 0) {
+            p.ty = std::min(p.ty, tile_y);
+            if (p.ty < std::min(tile_y, nl) && w + wps <= Shape<T>::kComputeWarps) continue;  // a larger CTA holds the asked tile
+        }
+        p.ytiles     = (nl + p.ty - 1) / p.ty;
+        p.total_rows = 10 * p.ytiles * nl;
+        p.rows       = chunk_x > 0 ? std::min(chunk_x, p.total_rows) : (p.total_rows + sms - 1) / sms;
+        p.ctas       = (p.total_rows + p.rows - 1) / p.rows;
+        const double waves = static_cast<double>((p.ctas + sms - 1) / sms);
+        const double c     = waves * (p.rows + 1) * ((w + 3) / 4 * 4 + 5.0);
+        if (cost < 0.0 || c < cost) {
+            cost = c;
+            best = p;
+        }
+        if (strips > nl) break;  // one tile holds every line
+    }
+    return best;
+}
+
+template <typename T>
 int epsdivdiv_apply(const EddLaunch<T>& p, cudaStream_t stream)
 {
+    if (10LL * p.nl * p.nl * p.nr >= (1LL << 31)) return -6;  // the kernels index nodes in 32 bits
+    const int nrc = p.nr - 1;
+    if (p.diagonal) {
+        const int n = 10 * p.nl * p.nl * p.nr;
+        edd_diagonal_kernel<T><<<(n + 255) / 256, 256, 0, stream>>>(p, n, Decoder(p.nr), Decoder(p.nl));
+        note_launch();
+        return cudaGetLastError() == cudaSuccess ? 0 : -2;
+    }
+    if (nrc < 2 || nrc > 128 || (nrc & (nrc - 1)) != 0) return -3;
+    if (!p.lateral || !p.boundary) return -4;
+    const int sms = sm_count();
+    if (sms <= 0) return -1;
+    const EddPlan plan = edd_plan<T>(p.nl, p.nr, sms, p.tile_y, p.chunk_x);
+    if (plan.warps == 0) return -5;
     EddArgs<T> a;
     a.nl     = p.nl;
     a.nr     = p.nr;
-    a.coords = p.coords;
+    a.geo    = p.lateral;
     a.radii  = p.radii;
+    a.bdiag  = p.boundary;
     a.k      = p.k;
     a.kq0    = p.kq0;
     for (int c = 0; c < 3; ++c) {
         a.src[c] = p.src[c];
         a.dst[c] = p.dst[c];
     }
-    a.bc_cmb  = p.bc_cmb;
-    a.bc_surf = p.bc_surf;
-    a.add     = p.add;
-    a.err     = p.err;
-    // tile shape: TY node lines per CTA (TY + 1 warps), CX node rows per x chunk
-    a.ty = p.tile_y > 0 ? p.tile_y : std::min(MaxWarps<T>::value - 1, p.nl);
-    if (p.chunk_x > 0) {
-        a.cx = p.chunk_x;
-    } else {
-        // One CTA per SM: pick the x-chunk that minimises waves x steps per CTA.
-        static std::atomic<int> sm_count[kMaxDevices];
-        int                     dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -1;
-        int sms = sm_count[dev].load(std::memory_order_relaxed);
-        if (sms == 0) {
-            if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-            sm_count[dev].store(sms, std::memory_order_relaxed);
-        }
-        const int ytiles = (p.nl + a.ty - 1) / a.ty;
-        long      best   = -1;
-        for (int cx = 4; cx <= std::max(4, p.nl); ++cx) {
-            const long ctas  = 10L * ytiles * ((p.nl + cx - 1) / cx);
-            const long waves = (ctas + sms - 1) / sms;
-            const long cost  = waves * (cx + 1);
-            if (best < 0 || cost < best || (cost == best && cx > a.cx)) {
-                best = cost;
-                a.cx = cx;
-            }
-        }
-    }
-    if (a.ty + 1 > MaxWarps<T>::value) return -4;
-    if (10LL * p.nl * p.nl * p.nr >= (1LL << 31)) return -6;  // the kernel indexes nodes in 32 bits
-    return launch<T>(a, p.diagonal, stream);
+    a.bc_cmb     = p.bc_cmb;
+    a.bc_surf    = p.bc_surf;
+    a.err        = p.err;
+    a.warps      = plan.warps;
+    a.strips     = plan.strips;
+    a.ty         = plan.ty;
+    a.ytiles     = plan.ytiles;
+    a.rows       = plan.rows;
+    a.total_rows = plan.total_rows;
+    const size_t smem = edd_smem<T>(p.nr, plan.warps, plan.strips).total;
+    auto go = [&](auto q0, auto multi) {
+        constexpr bool Q = decltype(q0)::value, M = decltype(multi)::value;
+        return p.add ? launch_cfg<T, Q, M, true>(a, smem, plan.ctas, stream)
+                     : launch_cfg<T, Q, M, false>(a, smem, plan.ctas, stream);
+    };
+    using Yes = std::true_type;
+    using No  = std::false_type;
+    if (nrc < 32) return p.kq0 ? go(Yes{}, Yes{}) : go(No{}, Yes{});
+    return p.kq0 ? go(Yes{}, No{}) : go(No{}, No{});
 }
 
-template int epsdivdiv_apply<double>(const EddLaunch<double>&, cudaStream_t);
-template int epsdivdiv_apply<float>(const EddLaunch<float>&, cudaStream_t);
+template <typename T>
+size_t edd_lateral_values(int nl)
+{
+    return static_cast<size_t>(10) * (nl - 1) * nl * Shape<T>::kGeo;
+}
+
+template <typename T>
+int edd_lateral_table(int nl, const double* coords, T* out, cudaStream_t st)
+{
+    const int n = 10 * (nl - 1) * nl;
+    edd_lateral_kernel<T><<<(n + 127) / 128, 128, 0, st>>>(nl, coords, out);
+    note_launch();
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+template <typename T>
+int edd_boundary_table(int nl, int nr, const double* coords, const double* colgeo, const double* radgeo, const T* k,
+                       const T* kq0, T* out, cudaStream_t st)
+{
+    const int n = 2 * 10 * nl * nl;
+    edd_boundary_kernel<T><<<(n + 255) / 256, 256, 0, st>>>(nl, nr, coords, colgeo, radgeo, k, kq0, out);
+    note_launch();
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+#define TN_INST(T)                                                                                                   \
+    template EddPlan edd_plan<T>(int, int, int, int, int);                                                          \
+    template int epsdivdiv_apply<T>(const EddLaunch<T>&, cudaStream_t);                                             \
+    template size_t edd_lateral_values<T>(int);                                                                    \
+    template int edd_lateral_table<T>(int, const double*, T*, cudaStream_t);                                      \
+    template int edd_boundary_table<T>(int, int, const double*, const double*, const double*, const T*, const T*, T*, \
+                                       cudaStream_t);
+TN_INST(double)
+TN_INST(float)
+#undef TN_INST
 
 }  // namespace tn

@@ -58,22 +58,26 @@ std::unique_ptr<Shell> make_shell(int lat_level, int rad_level, int num_levels, 
             }
             dl->canon_lat = upload(canon);
         }
-        if (h.nl > 1) {
-            const size_t ncol = static_cast<size_t>(10) * (h.nl - 1) * (h.nl - 1) * 20;
-            dl->colgeo64.alloc(ncol * sizeof(double));
-            dl->colgeo32.alloc(ncol * sizeof(float));
-            if (column_geometry_table<double>(h.nl, dl->coords64.as<double>(), dl->colgeo64.as<double>(), nullptr) != 0 ||
-                column_geometry_table<float>(h.nl, dl->coords32.as<float>(), dl->colgeo32.as<float>(), nullptr) != 0)
-                throw Error(kErrCuda, "column geometry launch failed");
-            cuda_check(cudaDeviceSynchronize(), "column geometry");
-        }
-        if (h.nr > 1) {
-            dl->radgeo64.alloc(static_cast<size_t>(h.nr - 1) * 3 * sizeof(double));
-            dl->radgeo32.alloc(static_cast<size_t>(h.nr - 1) * 3 * sizeof(float));
-            if (radial_geometry_table<double>(h.nr, dl->radii64.as<double>(), dl->radgeo64.as<double>(), nullptr) != 0 ||
-                radial_geometry_table<float>(h.nr, dl->radii32.as<float>(), dl->radgeo32.as<float>(), nullptr) != 0)
-                throw Error(kErrCuda, "radial geometry launch failed");
-            cuda_check(cudaDeviceSynchronize(), "radial geometry");
+        {
+            const size_t nc = static_cast<size_t>(10) * (h.nl - 1) * (h.nl - 1) * 20, nrad = static_cast<size_t>(h.nr - 1) * 3;
+            auto         pad = [](size_t n) { return (n + 63) / 64 * 64; };  // tables start at multiples of 256 bytes
+            const size_t l64 = edd_lateral_values<double>(h.nl), l32 = edd_lateral_values<float>(h.nl);
+            dl->geo.alloc(sizeof(double) * (pad(nc) + pad(l64) + pad(nrad)) + sizeof(float) * (pad(nc) + pad(l32) + pad(nrad)));
+            dl->colgeo64  = dl->geo.as<double>();
+            dl->lateral64 = dl->colgeo64 + pad(nc);
+            dl->radgeo64  = dl->lateral64 + pad(l64);
+            dl->colgeo32  = reinterpret_cast<float*>(dl->radgeo64 + pad(nrad));
+            dl->lateral32 = dl->colgeo32 + pad(nc);
+            dl->radgeo32  = dl->lateral32 + pad(l32);
+            int rc = column_geometry_table<double>(h.nl, dl->coords64.as<double>(), dl->colgeo64, nullptr) |
+                     column_geometry_table<float>(h.nl, dl->coords32.as<float>(), dl->colgeo32, nullptr) |
+                     edd_lateral_table<double>(h.nl, dl->coords64.as<double>(), dl->lateral64, nullptr) |
+                     edd_lateral_table<float>(h.nl, dl->coords64.as<double>(), dl->lateral32, nullptr);
+            if (h.nr > 1)
+                rc |= radial_geometry_table<double>(h.nr, dl->radii64.as<double>(), dl->radgeo64, nullptr) |
+                      radial_geometry_table<float>(h.nr, dl->radii32.as<float>(), dl->radgeo32, nullptr);
+            if (rc != 0) throw Error(kErrCuda, "geometry table launch failed");
+            cuda_check(cudaDeviceSynchronize(), "geometry tables");
         }
         dl->iface.num_classes = static_cast<int>(h.dup_offset.size()) - 1;
         dl->iface.offset      = dl->dup_offset.as<int32_t>();
@@ -267,6 +271,7 @@ void EpsDivDivOp::prepare_fp32(cudaStream_t st)
             throw Error(kErrCuda, "conversion launch failed");
         k32 = std::move(b);
     }
+    if (selective) (void)boundary_table<float>(k32.as<float>(), st);
     prepare_penalty(st);
     cuda_check(cudaStreamSynchronize(st), "prepare fp32");
 }
@@ -382,6 +387,34 @@ void EpsDivDivOp::prepare_penalty(cudaStream_t st)
 }
 
 template <typename T>
+const T* EpsDivDivOp::boundary_table(const T* kk, cudaStream_t st)
+{
+    DevBuf& buf = std::is_same<T, double>::value ? bdiag64 : bdiag32;
+    if (buf.get() == nullptr) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        cuda_check(cudaStreamIsCapturing(st, &cap), "capture status");
+        if (cap != cudaStreamCaptureStatusNone)
+            throw Error(kErrState, "the operator's boundary table must be built before stream capture");
+        const DeviceLevel& L = lvl();
+        DevBuf             b(sizeof(T) * 8 * 2 * 10 * static_cast<size_t>(L.nl()) * L.nl());
+        if (edd_boundary_table<T>(L.nl(), L.nr(), L.coords<double>(), L.colgeo<double>(), L.radgeo<double>(),
+                                  q0 ? nullptr : kk, q0 ? kk : nullptr, b.as<T>(), st) != 0)
+            throw Error(kErrCuda, "boundary table launch failed");
+        cuda_check(cudaStreamSynchronize(st), "boundary table");
+        buf = std::move(b);
+    }
+    return buf.as<T>();
+}
+
+void EpsDivDivOp::prepare_boundary(cudaStream_t st)
+{
+    if (precision == 0)
+        (void)boundary_table<double>(k.as<double>(), st);
+    else
+        (void)boundary_table<float>(k.as<float>(), st);
+}
+
+template <typename T>
 void EpsDivDivOp::add_penalty(const T* const* src, T* const* dst, cudaStream_t st)
 {
     if (!penalty_active() || diagonal) return;
@@ -456,6 +489,10 @@ void EpsDivDivOp::apply_t(const T* const* src, T* const* dst, cudaStream_t st)
     p.nr     = L.nr();
     p.coords = L.coords<T>();
     p.radii  = L.radii<T>();
+    p.lateral = L.lateral<T>();
+    p.colgeo  = L.colgeo<T>();
+    p.radgeo  = L.radgeo<T>();
+    if (!diagonal) p.boundary = boundary_table<T>(kk, st);
     if (q0)
         p.kq0 = kk;
     else

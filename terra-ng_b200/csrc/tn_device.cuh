@@ -46,15 +46,16 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                  : "memory");
 }
 
+// One try, suspended by the hardware for a short while at most. No time hint: with one the wait sleeps on a coarse timer.
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity)
 {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(parity), "r"(100000u)
+        : "r"(smem_addr(bar)), "r"(parity)
         : "memory");
     return ok != 0;
 }
@@ -70,10 +71,12 @@ __device__ __forceinline__ uint64_t global_timer_ns()
 // on timeout; the caller records the error and stops using the buffer.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, uint64_t limit_ns = 1000000000ull)
 {
-    if (mbar_try_wait(bar, parity)) return true;
+    for (int i = 0; i < 32; ++i)
+        if (mbar_try_wait(bar, parity)) return true;
     const uint64_t t0 = global_timer_ns();
     while (true) {
-        if (mbar_try_wait(bar, parity)) return true;
+        for (int i = 0; i < 16; ++i)
+            if (mbar_try_wait(bar, parity)) return true;
         if (global_timer_ns() - t0 > limit_ns) return false;
     }
 }

@@ -20,6 +20,10 @@ struct EddLaunch {
     int      nl = 0, nr = 0;
     const T* coords = nullptr;  // (10, nl, nl, 3)
     const T* radii  = nullptr;  // (nr)
+    const T*    lateral  = nullptr;  // edd_lateral_table of the level
+    const T*    boundary = nullptr;  // edd_boundary_table of the coefficient
+    const T*    colgeo   = nullptr;  // column_geometry_table / radial_geometry_table (diagonal mode)
+    const T*    radgeo   = nullptr;
     const T* k      = nullptr;  // nodal coefficient (10, nl, nl, nr) or nullptr
     const T* kq0    = nullptr;  // cell coefficient (10, nl-1, nl-1, nr-1) or nullptr
     const T* src[3] = {nullptr, nullptr, nullptr};
@@ -32,6 +36,24 @@ struct EddLaunch {
 };
 template <typename T>
 int epsdivdiv_apply(const EddLaunch<T>& p, cudaStream_t stream);
+
+// Launch shape of the apply: compute warps and strips of a CTA, node lines it owns, and the split of the
+// flattened rows (diamond, tile, x) over CTAs. warps = 0 where no shape fits.
+struct EddPlan {
+    int warps = 0, strips = 0, ty = 0, ytiles = 0, rows = 0, total_rows = 0, ctas = 0;
+};
+template <typename T>
+EddPlan edd_plan(int nl, int nr, int sms, int tile_y, int chunk_x);
+
+// Set-up tables of the apply: the level's lateral geometry in the kernel's layout, and the boundary rows'
+// diagonals of a coefficient (2 x 10 nl^2 x 8 values).
+template <typename T>
+size_t edd_lateral_values(int nl);
+template <typename T>
+int edd_lateral_table(int nl, const double* coords, T* out, cudaStream_t st);
+template <typename T>
+int edd_boundary_table(int nl, int nr, const double* coords, const double* colgeo, const double* radgeo, const T* k,
+                       const T* kq0, T* out, cudaStream_t st);
 
 // backward of the apply with respect to per-cell log-viscosity (adjoint.cu):
 // grad[cell] (+)= lambda_e^T A_e(kq0[cell]) u_e

@@ -111,8 +111,11 @@ DevBuf upload(const std::vector<T>& v)
 struct DeviceLevel {
     ShellLevel host;
     DevBuf     coords64, coords32;  // (10, nl, nl, 3)
-    DevBuf     colgeo64, colgeo32;  // (10, nl-1, nl-1, 20) per-column wedge geometry
-    DevBuf     radgeo64, radgeo32;  // (nr-1, 3) per-radial-cell factors
+    // geometry tables in one allocation, per precision: wedge geometry of the columns (10, nl-1, nl-1, 20), lateral
+    // table of the matrix-free apply (edd_lateral_table), factors of the radial cells (nr-1, 3)
+    DevBuf     geo;
+    double *   colgeo64 = nullptr, *lateral64 = nullptr, *radgeo64 = nullptr;
+    float *    colgeo32 = nullptr, *lateral32 = nullptr, *radgeo32 = nullptr;
     DevBuf     radii64, radii32;    // (nr)
     DevBuf     owned_lat;           // (10, nl, nl) uint8
     DevBuf     dup_offset, dup_members;
@@ -135,7 +138,19 @@ struct DeviceLevel {
     const T* colgeo() const;
     template <typename T>
     const T* radgeo() const;
+    template <typename T>
+    const T* lateral() const;
 };
+template <>
+inline const double* DeviceLevel::lateral<double>() const
+{
+    return lateral64;
+}
+template <>
+inline const float* DeviceLevel::lateral<float>() const
+{
+    return lateral32;
+}
 template <>
 inline const double* DeviceLevel::coords<double>() const
 {
@@ -149,22 +164,22 @@ inline const float* DeviceLevel::coords<float>() const
 template <>
 inline const double* DeviceLevel::colgeo<double>() const
 {
-    return colgeo64.as<double>();
+    return colgeo64;
 }
 template <>
 inline const float* DeviceLevel::colgeo<float>() const
 {
-    return colgeo32.as<float>();
+    return colgeo32;
 }
 template <>
 inline const double* DeviceLevel::radgeo<double>() const
 {
-    return radgeo64.as<double>();
+    return radgeo64;
 }
 template <>
 inline const float* DeviceLevel::radgeo<float>() const
 {
-    return radgeo32.as<float>();
+    return radgeo32;
 }
 template <>
 inline const double* DeviceLevel::radii<double>() const
@@ -228,6 +243,7 @@ struct EpsDivDivOp : Operator {
     bool   q0 = false;
     bool   diagonal = false;
     int    tile_y = 0, chunk_x = 0;
+    DevBuf bdiag64, bdiag32;  // boundary rows' diagonals of k (edd_boundary_table), per apply precision
 
     // free slip on both boundaries: the orthonormal rotation modes as coefficients over the raw modes e_i x X
     // (evaluated from the coordinates by the kernels) and the scratch of the penalty dst += eps sum_i (n_i^T src) n_i
@@ -263,6 +279,10 @@ struct EpsDivDivOp : Operator {
     template <typename T>
     void vjp_logeta(const T* const* u, const T* const* lam, T* grad_cell, cudaStream_t st) const;
     // free-slip/free-slip null-space penalty (epsilon_divdiv_kerngen.hpp:324-445, :711-785)
+    // builds the boundary table of an apply in T with coefficient kk (synchronous; no-op once built)
+    template <typename T>
+    const T* boundary_table(const T* kk, cudaStream_t st);
+    void prepare_boundary(cudaStream_t st);  // the table of the operator's own precision
     bool penalty_active() const { return bc_cmb == 2 && bc_surf == 2; }
     void prepare_penalty(cudaStream_t st);  // orthonormalises the modes (synchronous); no-op unless active or done
     template <typename T>

@@ -178,3 +178,33 @@ def test_apply_is_deterministic(cuda, level):
         again = torch.full_like(src, float("nan"))
         op.apply(src, again)
         assert torch.equal(again, first)
+
+
+@pytest.mark.parametrize("lat,rad", [(0, 1), (1, 1), (2, 1), (1, 4), (5, 2), (3, 5), (2, 6), (4, 6), (1, 7)])
+@pytest.mark.parametrize("bcs", [(1, 2), (2, 1), (0, 0)])
+def test_lateral_and_radial_levels(cuda, lat, rad, bcs):
+    """Strips that share a warp, fill one or take several, tiles with a single line, and nodal / cell coefficients in
+    both precisions, Replace and Add. Tolerances as in the equal-level tests."""
+    import torch
+
+    sh = O.Shell(lat, rad)
+    rng = np.random.default_rng(100 * lat + 10 * rad + bcs[0])
+    X = sh.physical_coords()
+    k = np.exp(np.log(10.0) * np.sin(X @ np.array([1.3, -0.7, 2.1])))
+    kc = np.exp(rng.uniform(-2.0, 2.0, (10, sh.nl - 1, sh.nl - 1, sh.nr - 1)))
+    u = consistent(sh, rng.standard_normal(sh.vec_shape))
+    g = T.Shell(lat, rad)
+    for q0 in (False, True):
+        ref = O.EpsDivDiv(sh, **({"k_q0": kc} if q0 else {"k": k}), bc_cmb=bcs[0], bc_surface=bcs[1]).apply(u)
+        for dt, tol in ((torch.float64, TOL64), (torch.float32, TOL32)):
+            coef = torch.tensor(kc if q0 else k, dtype=dt, device=cuda)
+            op = T.EpsDivDiv(g, **({"k_cell": coef} if q0 else {"k": coef}), bc_cmb=bcs[0], bc_surface=bcs[1])
+            src = torch.tensor(u, dtype=dt, device=cuda)
+            dst = torch.full_like(src, float("nan"))
+            op.apply(src, dst)
+            assert rel_err(dst.double().cpu().numpy(), ref) < tol
+            op.set_modes(T.ADD, T.SKIP_COMMUNICATION)
+            part, acc = torch.zeros_like(src), src.clone()
+            op.apply(src, part)
+            op.apply(src, acc)
+            assert rel_err(acc.double().cpu().numpy(), (src + part).double().cpu().numpy()) < tol
