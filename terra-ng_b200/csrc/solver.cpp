@@ -694,6 +694,10 @@ StokesSolver::StokesSolver(const Shell* sh, int vlevel, const double* eta_nodal,
     K_.B.scratch.alloc(wedges);
     K_.BT.scratch.alloc(wedges);
     BT_.scratch.alloc(wedges);
+    gs_partials_.alloc(sizeof(double) * gram_schmidt_partials(o.restart));
+    gram_.alloc(sizeof(double) * o.restart * o.restart);
+    owned_mask_.alloc(sizeof(uint64_t) * (blk_.total / 64));
+    chk(owned_mask(blk_, owned_mask_.as<uint64_t>(), st), "owned mask");
     graphs_.assign(o.restart, nullptr);
     graph_kernels_.assign(o.restart, 0);
     cuda_check(cudaStreamCreateWithFlags(&ws_, cudaStreamNonBlocking), "create stream");
@@ -858,12 +862,13 @@ void StokesSolver::arnoldi_tail(int j, cudaStream_t st)
 {
     stokes_apply(Z_[j], w_, st);
     if (opt_.project_pressure_mean) remove_pressure_mean(w_, kProj, st);
-    for (int i = 0; i <= j; ++i)
-        chk(mgs_step(blk_, w_.data(), i > 0 ? V_[i - 1].data() : nullptr, scratch_.s(kH0 + i - 1), V_[i].data(),
-                     scratch_.s(kH0 + i), scratch_.rs(), st),
-            "gram-schmidt");
-    chk(mgs_step(blk_, w_.data(), V_[j].data(), scratch_.s(kH0 + j), nullptr, scratch_.s(kH0 + j + 1), scratch_.rs(),
-                 st),
+    BasisList B;
+    B.m = j + 1;
+    for (int i = 0; i <= j; ++i) B.v[i] = V_[i].data();
+    RedScratch rs = scratch_.rs();
+    rs.partials   = gs_partials_.as<double>();
+    chk(gram_schmidt(blk_, owned_mask_.as<uint64_t>(), w_.data(), B, gram_.as<double>(), opt_.restart,
+                     scratch_.s(kH0), scratch_.s(kH0 + j + 1), rs, st),
         "gram-schmidt");
 }
 

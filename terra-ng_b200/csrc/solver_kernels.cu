@@ -4,9 +4,8 @@
 //   components (velocity on level L, pressure on level L-1), reduced in a fixed
 //   order by the last block to finish (no second launch, bitwise reproducible),
 //   with the result left in device memory so that the host does not wait.
-// * The FGMRES modified Gram-Schmidt step fused into one pass: w -= h_{i-1}
-//   v_{i-1} followed by h_i = <w, v_i> (fgmres.hpp:230-240 does the same
-//   arithmetic as two launches per basis vector, dot then lincomb).
+// * The FGMRES modified Gram-Schmidt of one iteration in two passes over the basis
+//   (fgmres.hpp:230-240 takes two launches per basis vector, dot then lincomb).
 // * The Chebyshev-Jacobi update d = alpha D^-1 (b - A x) + beta d, x += d in one
 //   pass (chebyshev.hpp:102-176 uses four BLAS-1 launches per step).
 // * The coarsest-grid CG (pcg.hpp:81-169, identity preconditioner) as a single
@@ -93,105 +92,193 @@ __global__ void __launch_bounds__(kThreads) vdot_kernel(VecDesc L, const T* __re
     block_finish(acc, rs, out, take_sqrt);
 }
 
-// L2 residency of the Gram-Schmidt target. One Arnoldi step reads and writes
-// w once per basis vector; w (the level-6 Stokes vector is 69 MB) fits in the
-// 126 MB L2 while the basis vectors stream past it. w is loaded and stored
-// with an evict_last policy and the basis vectors with streaming loads, so
-// each step reads the two basis vectors it uses (v_{i-1}, partly still in L2
-// from the step before, and v_i) from DRAM, instead of those two plus w read
-// and written. The last step of an Arnoldi iteration (the norm) stores w
-// with evict_normal, which hands the lines back to ordinary replacement before
-// the preconditioner runs.
-__device__ __forceinline__ uint64_t l2_policy(bool keep)
-{
-    uint64_t p;
-    if (keep)
-        asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-    else
-        asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
+// ---------------------------------------------------------------------------
+// Gram-Schmidt of w against the m = j + 1 basis vectors v_0 .. v_j in two passes.
+//
+// Modified Gram-Schmidt (fgmres.hpp:230-240) is h_i = <w_i, v_i>, w_{i+1} = w_i - h_i v_i. Since
+// w_i = w - sum_{k<i} h_k v_k, its coefficients solve the unit lower triangular system
+//   h_i = <w, v_i> - sum_{k<i} <v_k, v_i> h_k
+// with the basis vectors' own inner products (Swirydowicz, Langou, Ananthan, Yang, Thomas: Low synchronization
+// Gram-Schmidt and GMRES algorithms, Numer. Linear Algebra Appl. 2021). Pass 1 takes all <w, v_i> and the new row
+// <v_j, v_k> of that matrix together; its last block solves for h. Pass 2 subtracts sum h_i v_i in order and takes
+// the norm. Each basis vector is read twice per iteration, as in the vector-by-vector form, but w and v_j once per pass
+// instead of w once per vector, and 2 launches replace m + 1.
+//
+// What bounds it: the DRAM reads of the basis. A lane takes four 16-byte pieces of two basis vectors at a time, all
+// loaded before use. The inner products of a warp's 256 entries are reduced at once (two vectors share the shuffles) and
+// summed per warp in shared memory, then per block and over blocks in index order: results are reproducible. One
+// 64-bit word per 64 entries says which are owned (components start at multiples of 64 entries).
+// ---------------------------------------------------------------------------
+constexpr int kGsBlocks = 296;  // 2 x 148 SMs
+constexpr int kGsWarps  = kThreads / 32;
+constexpr int kGsPieces = 4;
 
-__device__ __forceinline__ double2 ld_policy(const double2* a, uint64_t pol)
+__global__ void owned_mask_kernel(VecDesc L, uint64_t* __restrict__ mask, int64_t words)
 {
-    double2 v;
-    asm volatile("ld.global.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(a), "l"(pol));
-    return v;
-}
-
-__device__ __forceinline__ void st_policy(double2* a, double2 v, uint64_t pol)
-{
-    asm volatile("st.global.L2::cache_hint.v2.f64 [%0], {%1, %2}, %3;" ::"l"(a), "d"(v.x), "d"(v.y), "l"(pol)
-                 : "memory");
-}
-
-// Gram-Schmidt step over pairs of entries (components start at multiples of
-// 64 entries, so pairs are 16-byte aligned); the odd tail entry is handled
-// by the thread that owns pair index n / 2. Each thread takes kMgsUnroll
-// grid-strided pairs per trip and issues all their loads before the first
-// store, so that enough bytes are in flight to cover DRAM latency; the pairs
-// are accumulated in the same order as a one-pair loop would.
-constexpr int kMgsUnroll = 2;
-
-// kSub: subtract h v_sub from w first (every step but the first);
-// kDot: dot with v_dot (every step but the last, which takes ||w||^2).
-template <bool kSub, bool kDot>
-__global__ void __launch_bounds__(kThreads) mgs_kernel(VecDesc L, double* __restrict__ w,
-                                                        const double* __restrict__ vsub, const double* hsub,
-                                                        const double* __restrict__ vdot, RedScratch rs, double* out,
-                                                        int take_sqrt)
-{
-    const double   h      = kSub ? *hsub : 0.0;
-    const uint64_t pol    = l2_policy(kDot);
-    double         acc    = 0.0;
-    const int64_t  stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int s = 0; s < L.nseg; ++s) {
-        const VecSeg  S  = L.seg[s];
-        const int64_t np = S.n / 2;
-        for (int c = 0; c < S.ncomp; ++c) {
-            const int64_t  o  = S.offset + c * S.stride;
-            double2*       w2 = reinterpret_cast<double2*>(w + o);
-            const double2* s2 = reinterpret_cast<const double2*>(vsub + o);
-            const double2* d2 = reinterpret_cast<const double2*>(vdot + o);
-            for (int64_t k0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k0 < np;
-                 k0 += kMgsUnroll * stride) {
-                double2 wv[kMgsUnroll], sv[kMgsUnroll], dv[kMgsUnroll];
-#pragma unroll
-                for (int u = 0; u < kMgsUnroll; ++u) {
-                    const int64_t k = k0 + u * stride;
-                    if (k < np) {
-                        wv[u] = ld_policy(w2 + k, pol);
-                        if constexpr (kSub) sv[u] = __ldcs(s2 + k);
-                        if constexpr (kDot) dv[u] = __ldcs(d2 + k);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < kMgsUnroll; ++u) {
-                    const int64_t k = k0 + u * stride;
-                    if (k < np) {
-                        if constexpr (kSub) {
-                            wv[u].x = wv[u].x - h * sv[u].x;
-                            wv[u].y = wv[u].y - h * sv[u].y;
-                            st_policy(w2 + k, wv[u], pol);
-                        }
-                        const double2 d = kDot ? dv[u] : wv[u];
-                        if (S.owned[lat_of(2 * k, S.rdiv)]) acc += wv[u].x * d.x;
-                        if (S.owned[lat_of(2 * k + 1, S.rdiv)]) acc += wv[u].y * d.y;
-                    }
-                }
-            }
-            if ((S.n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
-                const int64_t i  = S.n - 1;
-                double        wi = w[o + i];
-                if constexpr (kSub) {
-                    wi       = wi - h * vsub[o + i];
-                    w[o + i] = wi;
-                }
-                if (S.owned[lat_of(i, S.rdiv)]) acc += wi * (kDot ? vdot[o + i] : wi);
-            }
+    const int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k >= words) return;
+    uint64_t m = 0;
+    for (int b = 0; b < 64; ++b) {
+        const int64_t e = k * 64 + b;
+        for (int s = 0; s < L.nseg; ++s) {
+            const VecSeg& S = L.seg[s];
+            if (e < S.offset || e >= S.offset + S.ncomp * S.stride) continue;
+            const int64_t i = (e - S.offset) % S.stride;
+            if (i < S.n && S.owned[i / S.nr]) m |= uint64_t(1) << b;
         }
     }
-    block_finish(acc, rs, out, take_sqrt);
+    mask[k] = m;
+}
+
+__device__ __forceinline__ double2 masked(double2 v, uint64_t word, int lane)
+{
+    const uint32_t bits = static_cast<uint32_t>(word >> (2 * lane)) & 3u;
+    return make_double2((bits & 1u) ? v.x : 0.0, (bits & 2u) ? v.y : 0.0);
+}
+
+__global__ void __launch_bounds__(kThreads, 2) gs_dots_kernel(int64_t words, const uint64_t* __restrict__ mask,
+                                                              const double* __restrict__ w, BasisList B,
+                                                              RedScratch rs, double* gram, int ld, double* h)
+{
+    __shared__ double acc[kGsWarps][2 * kMaxAxpy];  // [2 i]: <w, v_i>, [2 i + 1]: <v_j, v_i>
+    __shared__ double hs;
+    __shared__ int    is_last;
+    const int     lane = threadIdx.x & 31, warp = threadIdx.x >> 5, m = B.m;
+    const double* vj   = B.v[m - 1];
+    for (int i = lane; i < 2 * m; i += 32) acc[warp][i] = 0.0;
+    __syncwarp();
+    const int64_t chunks = (words + kGsPieces - 1) / kGsPieces;
+    for (int64_t c = static_cast<int64_t>(blockIdx.x) * kGsWarps + warp; c < chunks;
+         c += static_cast<int64_t>(kGsBlocks) * kGsWarps) {
+        const int64_t first = c * kGsPieces, e = first * 64 + 2 * lane;
+        double2       wm[kGsPieces], jm[kGsPieces];
+#pragma unroll
+        for (int u = 0; u < kGsPieces; ++u) {
+            wm[u] = jm[u] = make_double2(0.0, 0.0);
+            if (first + u < words) {
+                const uint64_t bits = mask[first + u];
+                wm[u] = masked(*reinterpret_cast<const double2*>(w + e + 64 * u), bits, lane);
+                jm[u] = masked(*reinterpret_cast<const double2*>(vj + e + 64 * u), bits, lane);
+            }
+        }
+        for (int i = 0; i < m; i += 2) {
+            const double* p0 = B.v[i] + e;
+            const double* p1 = B.v[i + 1 < m ? i + 1 : i] + e;
+            double2       a0[kGsPieces], a1[kGsPieces];
+#pragma unroll
+            for (int u = 0; u < kGsPieces; ++u) {
+                a0[u] = a1[u] = make_double2(0.0, 0.0);
+                if (first + u < words) {
+                    a0[u] = *reinterpret_cast<const double2*>(p0 + 64 * u);
+                    a1[u] = *reinterpret_cast<const double2*>(p1 + 64 * u);
+                }
+            }
+            double t0 = 0.0, t1 = 0.0, g0 = 0.0, g1 = 0.0;
+#pragma unroll
+            for (int u = 0; u < kGsPieces; ++u) {
+                t0 = fma(wm[u].y, a0[u].y, fma(wm[u].x, a0[u].x, t0));
+                g0 = fma(jm[u].y, a0[u].y, fma(jm[u].x, a0[u].x, g0));
+                t1 = fma(wm[u].y, a1[u].y, fma(wm[u].x, a1[u].x, t1));
+                g1 = fma(jm[u].y, a1[u].y, fma(jm[u].x, a1[u].x, g1));
+            }
+            // lanes 0-15 go on with t, 16-31 with g; then bit 3 selects the vector
+            const bool hi = lane & 16, second = lane & 8;
+            double     k0 = hi ? g0 : t0, k1 = hi ? g1 : t1;
+            k0 += __shfl_xor_sync(0xffffffffu, hi ? t0 : g0, 16);
+            k1 += __shfl_xor_sync(0xffffffffu, hi ? t1 : g1, 16);
+            double k = second ? k1 : k0;
+            k += __shfl_xor_sync(0xffffffffu, second ? k0 : k1, 8);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
+            const int idx = 2 * (i + (second ? 1 : 0)) + (hi ? 1 : 0);
+            if ((lane & 7) == 0 && idx < 2 * m) acc[warp][idx] += k;
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * m; i += kThreads) {
+        double s = 0.0;
+        for (int k = 0; k < kGsWarps; ++k) s += acc[k][i];
+        rs.partials[static_cast<int64_t>(i) * kGsBlocks + blockIdx.x] = s;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) is_last = atomicAdd(rs.counter, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    for (int i = warp; i < 2 * m; i += kGsWarps) {
+        double s = 0.0;
+        for (int k = lane; k < kGsBlocks; k += 32) s += __ldcg(rs.partials + static_cast<int64_t>(i) * kGsBlocks + k);
+        s = warp_sum(s);
+        if (lane == 0) acc[0][i] = s;
+    }
+    __syncthreads();
+    // row j of the inner products, then forward substitution: thread k holds h_k once all h_i, i < k, are subtracted
+    const int k = threadIdx.x;
+    if (k < m - 1) gram[static_cast<int64_t>(m - 1) * ld + k] = acc[0][2 * k + 1];
+    double hk = k < m ? acc[0][2 * k] : 0.0;
+    for (int i = 0; i < m; ++i) {
+        const double g = (k > i && k < m) ? (k == m - 1 ? acc[0][2 * i + 1] : __ldcg(gram + static_cast<int64_t>(k) * ld + i)) : 0.0;
+        if (k == i) hs = hk;
+        __syncthreads();
+        if (k > i) hk -= hs * g;
+        __syncthreads();
+    }
+    if (k < m) h[k] = hk;
+    if (k == 0) *rs.counter = 0u;
+}
+
+// w -= sum h_i v_i in index order, *out = ||w||. Walks the entries from the end, where pass 1 stopped and the
+// basis is still in L2.
+__global__ void __launch_bounds__(kThreads, 2) gs_update_kernel(int64_t words, const uint64_t* __restrict__ mask,
+                                                                double* __restrict__ w, BasisList B, const double* h,
+                                                                RedScratch rs, double* out)
+{
+    __shared__ double hs[kMaxAxpy];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, m = B.m;
+    for (int i = threadIdx.x; i < m; i += kThreads) hs[i] = h[i];
+    __syncthreads();
+    double        acc    = 0.0;
+    const int64_t chunks = (words + kGsPieces - 1) / kGsPieces;
+    for (int64_t c = chunks - 1 - (static_cast<int64_t>(blockIdx.x) * kGsWarps + warp); c >= 0;
+         c -= static_cast<int64_t>(kGsBlocks) * kGsWarps) {
+        const int64_t first = c * kGsPieces, e = first * 64 + 2 * lane;
+        double2       v[kGsPieces];
+#pragma unroll
+        for (int u = 0; u < kGsPieces; ++u)
+            if (first + u < words) v[u] = *reinterpret_cast<const double2*>(w + e + 64 * u);
+        for (int i = 0; i < m; i += 2) {
+            const bool    two = i + 1 < m;
+            const double* p0  = B.v[i] + e;
+            const double* p1  = B.v[two ? i + 1 : i] + e;
+            const double  h0 = hs[i], h1 = two ? hs[i + 1] : 0.0;
+            double2       a0[kGsPieces], a1[kGsPieces];
+#pragma unroll
+            for (int u = 0; u < kGsPieces; ++u)
+                if (first + u < words) {
+                    a0[u] = *reinterpret_cast<const double2*>(p0 + 64 * u);
+                    if (two) a1[u] = *reinterpret_cast<const double2*>(p1 + 64 * u);
+                }
+#pragma unroll
+            for (int u = 0; u < kGsPieces; ++u)
+                if (first + u < words) {
+                    v[u].x = v[u].x - h0 * a0[u].x;
+                    v[u].y = v[u].y - h0 * a0[u].y;
+                    if (two) {
+                        v[u].x = v[u].x - h1 * a1[u].x;
+                        v[u].y = v[u].y - h1 * a1[u].y;
+                    }
+                }
+        }
+#pragma unroll
+        for (int u = 0; u < kGsPieces; ++u)
+            if (first + u < words) {
+                *reinterpret_cast<double2*>(w + e + 64 * u) = v[u];
+                const double2 q = masked(v[u], mask[first + u], lane);
+                acc             = fma(q.y, q.y, fma(q.x, q.x, acc));
+            }
+    }
+    block_finish(acc, rs, out, 1);
 }
 
 // CG update x += alpha p, r -= alpha ap with alpha = s_an / s_ad from device
@@ -915,18 +1002,23 @@ int vec_dot(const VecDesc& L, const T* a, const T* b, double* out_dev, RedScratc
 template int vec_dot<double>(const VecDesc&, const double*, const double*, double*, RedScratch, bool, cudaStream_t);
 template int vec_dot<float>(const VecDesc&, const float*, const float*, double*, RedScratch, bool, cudaStream_t);
 
-int mgs_step(const VecDesc& L, double* w, const double* v_sub, const double* h_sub, const double* v_dot, double* out,
-             RedScratch rs, cudaStream_t st)
+int owned_mask(const VecDesc& L, uint64_t* mask, cudaStream_t st)
 {
-    if (v_sub && v_dot)
-        mgs_kernel<true, true><<<kBlocks, kThreads, 0, st>>>(L, w, v_sub, h_sub, v_dot, rs, out, 0);
-    else if (v_dot)
-        mgs_kernel<false, true><<<kBlocks, kThreads, 0, st>>>(L, w, v_sub, h_sub, v_dot, rs, out, 0);
-    else if (v_sub)
-        mgs_kernel<true, false><<<kBlocks, kThreads, 0, st>>>(L, w, v_sub, h_sub, v_dot, rs, out, 1);
-    else
-        mgs_kernel<false, false><<<kBlocks, kThreads, 0, st>>>(L, w, v_sub, h_sub, v_dot, rs, out, 1);
+    const int64_t words = L.total / 64;
+    owned_mask_kernel<<<static_cast<unsigned>((words + 255) / 256), 256, 0, st>>>(L, mask, words);
     return launch_status();
+}
+
+int64_t gram_schmidt_partials(int max_basis) { return 2 * static_cast<int64_t>(max_basis) * kGsBlocks; }
+
+int gram_schmidt(const VecDesc& L, const uint64_t* mask, double* w, const BasisList& B, double* gram, int ld, double* h,
+                 double* norm, RedScratch rs, cudaStream_t st)
+{
+    if (B.m < 1 || B.m > kMaxAxpy || L.total % 64 != 0) return -1;
+    const int64_t words = L.total / 64;
+    gs_dots_kernel<<<kGsBlocks, kThreads, 0, st>>>(words, mask, w, B, rs, gram, ld, h);
+    gs_update_kernel<<<kGsBlocks, kThreads, 0, st>>>(words, mask, w, B, h, rs, norm);
+    return launch_status(2);
 }
 
 int cg_update(const VecDesc& L, double* x, double* r, const double* p, const double* ap, const double* s_an,

@@ -310,9 +310,18 @@ struct CoarsePcgArgs {
 int solver_partials_size();
 template <typename T>
 int vec_dot(const VecDesc& L, const T* a, const T* b, double* out_dev, RedScratch rs, bool take_sqrt, cudaStream_t st);
-// w -= (*h_sub) v_sub (when v_sub), then *out = <w, v_dot> or ||w|| (v_dot == nullptr)
-int mgs_step(const VecDesc& L, double* w, const double* v_sub, const double* h_sub, const double* v_dot, double* out,
-             RedScratch rs, cudaStream_t st);
+// Modified Gram-Schmidt of w against basis vectors v_0 .. v_{m-1} (1 <= m <= kMaxAxpy): h[i] its coefficients,
+// w the remainder, *norm = ||w|| (owned entries). gram (ld x ld) keeps the basis vectors' inner products between the
+// calls of one cycle, row m - 1 added by each call; mask = owned_mask of the layout; rs.partials holds
+// gram_schmidt_partials(m) doubles.
+struct BasisList {
+    const double* v[kMaxAxpy];
+    int           m = 0;
+};
+int     owned_mask(const VecDesc& L, uint64_t* mask, cudaStream_t st);  // one bit per entry, L.total / 64 words
+int64_t gram_schmidt_partials(int max_basis);
+int     gram_schmidt(const VecDesc& L, const uint64_t* mask, double* w, const BasisList& B, double* gram, int ld, double* h,
+                     double* norm, RedScratch rs, cudaStream_t st);
 // x += a p, r -= a ap with a = *s_an / *s_ad; *out = ||r|| (or -1 when
 // |*s_ad| < DBL_MIN, in which case nothing is updated)
 int cg_update(const VecDesc& L, double* x, double* r, const double* p, const double* ap, const double* s_an,

@@ -180,6 +180,7 @@ class StokesSolver {
     StokesOp                           K_;
     GradientOp                         BT_;
     DVec<double>                       inv_schur_;  // pressure level
+    DevBuf                             gs_partials_, gram_, owned_mask_;  // Gram-Schmidt (gram_schmidt)
     DVec<double>                       ones_p_;     // pressure level, for the mean
     int64_t                            num_owned_p_ = 0;
     std::unique_ptr<VelocityMultigrid> mg_;
