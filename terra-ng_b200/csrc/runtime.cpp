@@ -282,21 +282,27 @@ void EpsDivDivOp::ensure_baked(bool need32, cudaStream_t st)
     const DevBuf&      src = selective ? sel_delta : mats;
     if (selective ? !sel_built : (!stored || mats.get() == nullptr))
         throw Error(kErrState, "stored matrix mode without matrices");
-    const size_t nv = static_cast<size_t>(mats_values());
+    const size_t nv = static_cast<size_t>(baked_values());
     if (nv == 0) return;
     if (baked_bc[0] != bc_cmb || baked_bc[1] != bc_surf || baked64.get() == nullptr) {
-        if (baked64.get() == nullptr) baked64.alloc(nv * sizeof(double));
-        cuda_check(cudaMemcpyAsync(baked64.get(), src.get(), nv * sizeof(double), cudaMemcpyDeviceToDevice, st),
-                   "copy matrices");
-        if (gca_bake_boundary(L.nl(), L.nr(), L.coords<double>(), L.radii<double>(), bc_cmb, bc_surf,
-                              baked64.as<double>(), st, selective ? sel_cells.as<int>() : nullptr, sel_count) != 0)
-            throw Error(kErrCuda, "boundary bake launch failed");
+        baked64.ensure(nv * sizeof(double));
+        if (compact()) {
+            if (gca_compact(L.nl(), L.nr(), L.coords<double>(), L.radii<double>(), bc_cmb, bc_surf, src.as<double>(),
+                            baked64.as<double>(), st) != 0)
+                throw Error(kErrCuda, "compact store launch failed");
+        } else {
+            cuda_check(cudaMemcpyAsync(baked64.get(), src.get(), nv * sizeof(double), cudaMemcpyDeviceToDevice, st),
+                       "copy matrices");
+            if (gca_bake_boundary(L.nl(), L.nr(), L.coords<double>(), L.radii<double>(), bc_cmb, bc_surf,
+                                  baked64.as<double>(), st, selective ? sel_cells.as<int>() : nullptr, sel_count) != 0)
+                throw Error(kErrCuda, "boundary bake launch failed");
+        }
         baked_bc[0]   = bc_cmb;
         baked_bc[1]   = bc_surf;
         baked32_valid = false;
     }
     if (need32 && !baked32_valid) {
-        if (baked32.get() == nullptr) baked32.alloc(nv * sizeof(float));
+        baked32.ensure(nv * sizeof(float));
         if (gca_to_f32(static_cast<int64_t>(nv), baked64.as<double>(), baked32.as<float>(), st) != 0)
             throw Error(kErrCuda, "matrix conversion launch failed");
         baked32_valid = true;
@@ -472,7 +478,8 @@ void EpsDivDivOp::apply_t(const T* const* src, T* const* dst, cudaStream_t st)
             ensure_baked(std::is_same<T, float>::value, st);
             const T* m = std::is_same<T, float>::value ? static_cast<const T*>(baked32.get())
                                                        : static_cast<const T*>(baked64.get());
-            if (gca_apply_add<T>(L.nl(), L.nr(), m, src, dst, st) != 0)
+            if ((compact() ? gca_apply_compact_add<T>(L.nl(), L.nr(), m, src, dst, st)
+                           : gca_apply_add<T>(L.nl(), L.nr(), m, src, dst, st)) != 0)
                 throw Error(kErrCuda, "stored apply launch failed");
             add_penalty<T>(src, dst, st);
         }

@@ -210,6 +210,7 @@ VelocityMultigrid::VelocityMultigrid(const Shell* sh, const EpsDivDivOp& fine, c
     // the coarsest CG runs over stored matrices
     ops64_[0]->materialize_full(st);
     if (!ops64_[0]->stored) ops64_[0]->set_stored_matrices_from_coefficient(st);
+    ops64_[0]->packed_layout = true;
     ops64_[0]->ensure_baked(false, st);
     {
         const DeviceLevel& L0   = sh->level(0);

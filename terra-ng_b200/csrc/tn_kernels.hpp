@@ -214,6 +214,13 @@ int gca_mark_elements(int nl, int nr, const double* k, int level_range, uint8_t*
 int gca_bake_boundary(int nl, int nr, const double* coords, const double* radii, int bc_cmb, int bc_surf, double* mats,
                       cudaStream_t st, const int* cells = nullptr, int nslots = 0);
 // dst += A src with baked matrices
+// Compact store of all cells of a level for the apply (gca.cu), boundary conditions baked in: gca_compact_values
+// doubles, built from the packed matrices [342][cells].
+int64_t gca_compact_values(int nl, int nr);
+int     gca_compact(int nl, int nr, const double* coords, const double* radii, int bc_cmb, int bc_surf, const double* mats,
+                    double* out, cudaStream_t st);
+template <typename T>
+int gca_apply_compact_add(int nl, int nr, const T* mats, const T* const* src, T* const* dst, cudaStream_t st);
 template <typename T>
 int gca_apply_add(int nl, int nr, const T* mats, const T* const* src, T* const* dst, cudaStream_t st,
                   const int* cells = nullptr, int nslots = 0);

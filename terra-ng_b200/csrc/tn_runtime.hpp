@@ -253,7 +253,10 @@ struct EpsDivDivOp : Operator {
 
     bool   stored = false;
     DevBuf mats;              // FP64 unbaked element matrices [342][cells] ([342][sel_count] when selective)
-    DevBuf baked64, baked32;  // boundary-baked copies (built lazily; of sel_delta when selective)
+    // boundary-baked copies (built lazily): a compact store of mats, or packed copies of sel_delta (selective) and of
+    // mats where packed_layout asks for them (the coarsest level, whose CG reads packed matrices)
+    DevBuf baked64, baked32;
+    bool   packed_layout = false;
     int    baked_bc[2]   = {-1, -1};
     bool   baked32_valid = false;
 
@@ -291,6 +294,8 @@ struct EpsDivDivOp : Operator {
     void ensure_baked(bool need32, cudaStream_t st);
     void set_stored_matrices_from_coefficient(cudaStream_t st);  // element matrices of this level
     int64_t mats_values() const;  // FP64 values of mats
+    bool    compact() const { return !selective && !packed_layout; }
+    int64_t baked_values() const { return compact() ? gca_compact_values(lvl().nl(), lvl().nr()) : mats_values(); }
     // selective storage: cells whose ancestor level_range levels down is marked in marks_dev (one byte per cell
     // of that level) get stored matrices once a GCA build fills them (synchronous)
     void set_selective(const uint8_t* marks_dev, int level_range, cudaStream_t st);

@@ -546,3 +546,25 @@ def test_gram_schmidt_against_vector_by_vector(cuda, lat, rad, restart):
             xr = lin(xr, y[i], Z[i])
     assert len(hist) == len(ref)
     assert np.abs(np.array(hist) - np.array(ref)).max() < 1e-8
+
+
+@pytest.mark.parametrize("lat,rad", [(1, 1), (2, 1), (1, 4), (2, 2), (3, 3)])
+@pytest.mark.parametrize("bcs", [(1, 2), (0, 1), (2, 2)])
+def test_compact_store_radial_layers(cuda, lat, rad, bcs):
+    """Stored matrices without their null space: levels of two layers (edge cells only), three and more, and one wider
+    than a block. The stored element matrices give the matrix-free operator, in FP64 and, for the same matrices behind an
+    FP32 operator, in FP32; bounds as in the tests above. Rebuilding after a change of boundary conditions too."""
+    import torch
+
+    sh = O.Shell(lat, rad)
+    g = T.Shell(lat, rad)
+    k = smooth_viscosity(sh, 27, 100.0)
+    u = consistent(sh, O.seeded_normal(sh.vec_shape, 28))
+    op = T.EpsDivDiv(g, 0, k=_t(k), bc_cmb=bcs[0], bc_surface=bcs[1])
+    op.set_stored_matrix_mode(T.STORED_FULL)
+    out = torch.zeros(sh.vec_shape, dtype=torch.float64, device=cuda)
+    for b in (bcs, (1, 1), bcs):
+        op.set_boundary_conditions(*b)
+        op.apply(_t(u), out)
+        ref = O.EpsDivDiv(sh, k=k, bc_cmb=b[0], bc_surface=b[1]).apply(u, path="slow")
+        assert rel_err(out.cpu().numpy(), ref) < 1e-12
