@@ -140,6 +140,7 @@ struct GcaBuildArgs {
     int           nlf = 0, nrf = 0;     // fine level dims
     const double* coords    = nullptr;  // fine coords
     const double* radii     = nullptr;  // fine radii
+    const double* colgeo    = nullptr;  // fine column geometry (column_geometry_table; on-the-fly build)
     const double* k         = nullptr;  // fine nodal coefficient (on-the-fly matrices) or nullptr
     const double* kq0       = nullptr;  // fine cell coefficient or nullptr
     const double* fine_mats = nullptr;  // stored fine matrices [342][fine_stride] or nullptr
@@ -413,90 +414,167 @@ __global__ void __launch_bounds__(kMmaThreads) gca_build_mma_kernel(GcaBuildArgs
 // P_vec = I_3 (x) P the triple product keeps that form with the gradients replaced by h_c = sum_n P[n][c] g_n
 // (the coarse shape-function gradients seen from the fine wedge):
 // (P^T A_f P)[(c,a)][(e,b)] = kwJ (delta_ab h_c.h_e + h_c[b] h_e[a] - 2/3 h_c[a] h_e[b]).
-// Each fine wedge then costs 18 six-term sums and one rank-structured update of the 171 packed entries per
-// coarse wedge instead of two 18 x 18 x 6 products; exact in exact arithmetic, rounding differs from the
-// triple product in the last bits. The set-up is spread over the CTA in three short phases: the geometry of
-// the four fine columns and the 96 rows of the 16 interpolation matrices; the 16 x 18 gradients and the 16
-// weights; the 16 x 18 entries of h. Thread (t, p) of the first 342 then sums entry p of coarse wedge t over
-// the 8 fine wedges it receives.
-constexpr int kRankThreads = 352;
+// Exact in exact arithmetic, rounding differs from the triple product in the last bits.
+//
+// A CTA takes 32 consecutive slots, one per lane. First its 16 warps compute the gradients h and the weight of one
+// fine wedge each, for all 32 cells, into shared memory (values x lanes, no bank conflicts). Then warp (t, g) sums the
+// entries of two or three node pairs (c, e) of coarse wedge t over the 8 fine wedges it receives, in registers, and
+// writes them: 32 consecutive doubles per value. One CTA of 352 threads per coarse hex, which wrote 342 separate
+// doubles and went through three block barriers for one cell, took 6.4 ms for the 327,680 cells of level 5.
+constexpr int kRankCells  = 32;
+constexpr int kRankWarps  = 16;
+constexpr int kRankGroups = 8;
+constexpr size_t kRankSmem = sizeof(double) * (kFineWedges * 19 * kRankCells + 2 * kFineWedges * 36);
 
-__global__ void __launch_bounds__(kRankThreads, 3) gca_build_rank_kernel(GcaBuildArgs A)
+// node pair q (0 .. 20) of the upper triangle of the six nodes; group g holds pairs first(g) .. first(g + 1) - 1
+__host__ __device__ constexpr int rank_row(int q)
 {
-    const int nlf = A.nlf, nrf = A.nrf;
-    int       slot, d, xc, yc, rc;
-    if (!coarse_cell_of_block(A, slot, d, xc, yc, rc)) return;
+    int a = 0;
+    while (q >= 6 - a) {
+        q -= 6 - a;
+        ++a;
+    }
+    return a;
+}
+__host__ __device__ constexpr int rank_col(int q)
+{
+    int a = 0;
+    while (q >= 6 - a) {
+        q -= 6 - a;
+        ++a;
+    }
+    return a + q;
+}
+__host__ __device__ constexpr int rank_first(int g) { return g < 5 ? 3 * g : 2 * g + 5; }
 
-    __shared__ double Gw[4][20];  // column_geometry of fine column q = x + 2 y (both wedges)
-    __shared__ double P[kFineWedges][6][6];
-    __shared__ double G[kFineWedges][6][3];
-    __shared__ double H[kFineWedges][6][3];
-    __shared__ double kw[kFineWedges];
+// Sums of group G of coarse wedge t for the cell of this lane: H[f][3 node + comp][lane], weight in row 18.
+template <int G>
+__device__ __forceinline__ void rank_group(const double* H, int t, int lane, double* out, int64_t stride)
+{
+    constexpr int first = rank_first(G), count = rank_first(G + 1) - first;
+    double        acc[count][9] = {};
+    for (int f = 0; f < kFineWedges; ++f) {
+        if (target_wedge(f >> 1, f & 1) != t) continue;
+        const double* h  = H + f * 19 * kRankCells + lane;
+        const double  kw = h[18 * kRankCells];
+#pragma unroll
+        for (int k = 0; k < count; ++k) {
+            const int    c = rank_row(first + k), e = rank_col(first + k);
+            double       hc[3], he[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                hc[a] = kw * h[(3 * c + a) * kRankCells];
+                he[a] = h[(3 * e + a) * kRankCells];
+            }
+            const double dot = fma(hc[2], he[2], fma(hc[1], he[1], hc[0] * he[0]));
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    if (c == e && a > b) continue;
+                    if (a == b)
+                        acc[k][3 * a + b] += fma((1.0 / 3.0) * hc[a], he[a], dot);
+                    else
+                        acc[k][3 * a + b] = fma(hc[b], he[a], fma((-2.0 / 3.0) * hc[a], he[b], acc[k][3 * a + b]));
+                }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < count; ++k) {
+        const int c = rank_row(first + k), e = rank_col(first + k);
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                if (c == e && a > b) continue;
+                out[static_cast<int64_t>(t * kPack + pidx(c + 6 * a, e + 6 * b)) * stride] = acc[k][3 * a + b];
+            }
+    }
+}
 
-    const int tid = threadIdx.x;
-    if (tid < 4) {
-        column_geometry<double>(A.coords, nlf, d, 2 * xc + (tid & 1), 2 * yc + (tid >> 1), Gw[tid]);
-    } else if (tid >= 32 && tid < 32 + 6 * kFineWedges) {
-        const int f = (tid - 32) / 6, fl = (tid - 32) % 6;
+__global__ void __launch_bounds__(32 * kRankWarps) gca_build_rank_kernel(GcaBuildArgs A)
+{
+    extern __shared__ double smem[];
+    double*   H   = smem;                                     // [fine wedge][19][32]
+    double*   Pt  = smem + kFineWedges * 19 * kRankCells;     // constant interpolation [outer][fine wedge][6][6]
+    const int nlf = A.nlf, nrf = A.nrf, nlc = (nlf + 1) / 2, nrc = (nrf + 1) / 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int slot = blockIdx.x * kRankCells + lane;
+    const bool on  = slot < A.nout;
+    int        d, xc, yc, rc;
+    decode_cell(on ? (A.cells ? A.cells[slot] : slot) : 0, nlc, nrc, d, xc, yc, rc);
+    if (!A.linw && threadIdx.x < 2 * kFineWedges * 6) {
+        // rows of the 16 interpolation matrices of a coarse hex, inside the shell and on its outermost layer
+        const int outer = threadIdx.x / (kFineWedges * 6), f = threadIdx.x / 6 % kFineWedges, fl = threadIdx.x % 6;
         int       fx, fy, fr;
-        fine_hex(f >> 1, xc, yc, rc, fx, fy, fr);
-        interp_row(d, fx, fy, fr, f & 1, fl, nlf, nrf, A.linw, P[f][fl]);
+        fine_hex(f >> 1, 0, 0, 0, fx, fy, fr);
+        double row[6];
+        interp_row(0, fx, fy, fr, f & 1, fl, 3, outer ? 3 : 5, nullptr, row);
+        for (int c = 0; c < 6; ++c) Pt[(threadIdx.x / 6) * 36 + 6 * fl + c] = row[c];
     }
     __syncthreads();
-    if (tid < kFineWedges * 18) {
-        // gradient component c of shape function n of fine wedge f (as fine_wedge_factors)
-        const int     f = tid / 18, n = (tid % 18) / 3, c = tid % 3, h = f >> 1, w = f & 1;
-        const int     fr = 2 * rc + (h >> 2);
+    if (on) {
+        const int f = warp, w = f & 1;
+        int       fx, fy, fr;
+        fine_hex(f >> 1, xc, yc, rc, fx, fy, fr);
+        const double* gw = A.colgeo + ((static_cast<int64_t>(d) * (nlf - 1) + fx) * (nlf - 1) + fy) * 20 + 10 * w;
         const double  r0 = A.radii[fr], r1 = A.radii[fr + 1];
         const double  rm = 0.5 * (r0 + r1), hdr = 0.5 * (r1 - r0);
         const double  alpha = 0.5 / rm, beta = 1.0 / (6.0 * hdr);
-        const double* gw = Gw[h & 3] + 10 * w;
-        const int     m  = n % 3;
-        const double  sg = n < 3 ? -1.0 : 1.0;
-        const double  L  = m == 0 ? -(gw[c] + gw[3 + c]) : (m == 1 ? gw[c] : gw[3 + c]);
-        G[f][n][c]       = alpha * L + sg * beta * gw[6 + c];
-    } else if (tid >= 288 && tid < 288 + kFineWedges) {
-        const int f = tid - 288, h = f >> 1, w = f & 1;
-        int       fx, fy, fr;
-        fine_hex(h, xc, yc, rc, fx, fy, fr);
-        const double r0 = A.radii[fr], r1 = A.radii[fr + 1];
-        const double rm = 0.5 * (r0 + r1), hdr = 0.5 * (r1 - r0);
-        double       kv;
+        double        h[6][3] = {};
+        const double* P0 = Pt + (rc == nrc - 2 ? kFineWedges * 36 : 0) + f * 36;
+#pragma unroll
+        for (int n = 0; n < 6; ++n) {
+            double g[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double L = n % 3 == 0 ? -(gw[c] + gw[3 + c]) : (n % 3 == 1 ? gw[c] : gw[3 + c]);
+                g[c]           = alpha * L + (n < 3 ? -beta : beta) * gw[6 + c];
+            }
+            double row[6];
+            if (A.linw) {
+                interp_row(d, fx, fy, fr, w, n, nlf, nrf, A.linw, row);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 6; ++c) row[c] = P0[6 * n + c];
+            }
+#pragma unroll
+            for (int c = 0; c < 6; ++c)
+#pragma unroll
+                for (int a = 0; a < 3; ++a) h[c][a] = fma(row[c], g[a], h[c][a]);
+        }
+        double kv;
         if (A.kq0) {
             kv = A.kq0[node_index(nlf - 1, nrf - 1, d, fx, fy, fr)];
         } else {
             const double wlat0 = 1.0 - 1.0 / 3.0 - 1.0 / 3.0, wlat = 1.0 / 3.0;
             kv                 = 0.0;
+#pragma unroll
             for (int n = 0; n < 6; ++n)
                 kv += (n % 3 == 0 ? wlat0 : wlat) * 0.5 *
                       A.k[node_index(nlf, nrf, d, fx + woff(w, n, 0), fy + woff(w, n, 1), fr + woff(w, n, 2))];
         }
-        kw[f] = kv * Gw[h & 3][10 * w + 9] * rm * rm * hdr;
-    }
-    __syncthreads();
-    if (tid < kFineWedges * 18) {
-        const int f = tid / 18, c = (tid % 18) / 3, a = tid % 3;
-        double    h = 0.0;
+        double* o = H + f * 19 * kRankCells + lane;
 #pragma unroll
-        for (int n = 0; n < 6; ++n) h += P[f][n][c] * G[f][n][a];
-        H[f][c][a] = h;
+        for (int c = 0; c < 6; ++c)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) o[(3 * c + a) * kRankCells] = h[c][a];
+        o[18 * kRankCells] = kv * gw[9] * rm * rm * hdr;
     }
     __syncthreads();
-    if (tid >= 2 * kPack) return;
-    const int t = tid / kPack, p = tid % kPack;
-    int       i, j;
-    packed_pair(p, i, j);
-    const int ni = i % 6, di = i / 6, nj = j % 6, dj = j / 6;
-    double    acc = 0.0;
-    for (int f = 0; f < kFineWedges; ++f) {
-        if (target_wedge(f >> 1, f & 1) != t) continue;
-        const double* hi = H[f][ni];
-        const double* hj = H[f][nj];
-        double        v  = hi[dj] * hj[di] - (2.0 / 3.0) * hi[di] * hj[dj];
-        if (di == dj) v += hi[0] * hj[0] + hi[1] * hj[1] + hi[2] * hj[2];
-        acc += kw[f] * v;
+    if (!on) return;
+    const int t = warp / kRankGroups;
+    double*   out = A.out + slot;
+    switch (warp % kRankGroups) {
+    case 0: rank_group<0>(H, t, lane, out, A.nout); break;
+    case 1: rank_group<1>(H, t, lane, out, A.nout); break;
+    case 2: rank_group<2>(H, t, lane, out, A.nout); break;
+    case 3: rank_group<3>(H, t, lane, out, A.nout); break;
+    case 4: rank_group<4>(H, t, lane, out, A.nout); break;
+    case 5: rank_group<5>(H, t, lane, out, A.nout); break;
+    case 6: rank_group<6>(H, t, lane, out, A.nout); break;
+    default: rank_group<7>(H, t, lane, out, A.nout); break;
     }
-    A.out[static_cast<int64_t>(t * kPack + p) * A.nout + slot] = acc;
 }
 
 // Element matrices of one level itself (no coarsening): the stored form of the
@@ -1003,8 +1081,8 @@ int gca_values_per_cell() { return 2 * kPack; }
 namespace {
 constexpr int kMaxDevices = 64;  // devices a process can drive
 
-// the mma build's dynamic shared-memory limit, raised once per device
-int mma_smem_configure()
+// the dynamic shared-memory limits of the two builds, raised once per device
+int build_smem_configure()
 {
     static std::mutex mu;
     static bool       done[kMaxDevices] = {};
@@ -1013,7 +1091,9 @@ int mma_smem_configure()
     std::lock_guard<std::mutex> lock(mu);
     if (!done[dev]) {
         if (cudaFuncSetAttribute(gca_build_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kMmaSmem)) != cudaSuccess)
+                                 static_cast<int>(kMmaSmem)) != cudaSuccess ||
+            cudaFuncSetAttribute(gca_build_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(kRankSmem)) != cudaSuccess)
             return -1;
         done[dev] = true;
     }
@@ -1021,7 +1101,7 @@ int mma_smem_configure()
 }
 }  // namespace
 
-int gca_build(int nlf, int nrf, const double* coords_f, const double* radii_f, const double* k_f, const double* kq0_f,
+int gca_build(int nlf, int nrf, const double* coords_f, const double* radii_f, const double* colgeo_f, const double* k_f, const double* kq0_f,
               const double* fine_mats, double* coarse_mats, cudaStream_t st, const double* linear_weights,
               bool tensor_cores, const GcaSlots& sl)
 {
@@ -1046,9 +1126,11 @@ int gca_build(int nlf, int nrf, const double* coords_f, const double* radii_f, c
     if (!tensor_cores) {
         gca_build_kernel<<<a.nout, kN * kN, 0, st>>>(a);
     } else if (fine_mats == nullptr) {
-        gca_build_rank_kernel<<<a.nout, kRankThreads, 0, st>>>(a);
+        if (!colgeo_f || build_smem_configure() != 0) return -1;
+        a.colgeo = colgeo_f;
+        gca_build_rank_kernel<<<(a.nout + kRankCells - 1) / kRankCells, 32 * kRankWarps, kRankSmem, st>>>(a);
     } else {
-        if (mma_smem_configure() != 0) return -1;
+        if (build_smem_configure() != 0) return -1;
         gca_build_mma_kernel<<<a.nout, kMmaThreads, kMmaSmem, st>>>(a);
     }
     return launch_status();

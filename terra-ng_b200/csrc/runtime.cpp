@@ -338,7 +338,7 @@ void gca_coarsen(const EpsDivDivOp& fine, EpsDivDivOp& coarse, cudaStream_t st, 
     const double* kf         = (on_the_fly && !fine.q0) ? fine.k.as<double>() : nullptr;
     const double* kq0f       = (on_the_fly && fine.q0) ? fine.k.as<double>() : nullptr;
     const double* linw       = linear ? Lf.linear_weights<double>(st) : nullptr;
-    if (gca_build(Lf.nl(), Lf.nr(), Lf.coords<double>(), Lf.radii<double>(), kf, kq0f,
+    if (gca_build(Lf.nl(), Lf.nr(), Lf.coords<double>(), Lf.radii<double>(), Lf.colgeo<double>(), kf, kq0f,
                   on_the_fly ? nullptr : fine.mats.as<double>(), coarse.mats.as<double>(), st, linw, tensor_cores,
                   sl) != 0)
         throw Error(kErrCuda, "GCA build launch failed");

@@ -197,7 +197,7 @@ struct GcaSlots {
 // tensor_cores: the fast build -- over on-the-fly fine matrices the rank form of the triple product, over
 // stored ones the triple products as FP64 tensor-core tiles (mma m8n8k4); false: the plain scalar triple
 // product one fine wedge at a time.
-int gca_build(int nlf, int nrf, const double* coords_f, const double* radii_f, const double* k_f, const double* kq0_f,
+int gca_build(int nlf, int nrf, const double* coords_f, const double* radii_f, const double* colgeo_f, const double* k_f, const double* kq0_f,
               const double* fine_mats, double* coarse_mats, cudaStream_t st, const double* linear_weights = nullptr,
               bool tensor_cores = true, const GcaSlots& slots = GcaSlots{});
 // element matrices of a level (the stored form of the on-the-fly operator), of every cell or of the listed

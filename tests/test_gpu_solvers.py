@@ -568,3 +568,24 @@ def test_compact_store_radial_layers(cuda, lat, rad, bcs):
         op.apply(_t(u), out)
         ref = O.EpsDivDiv(sh, k=k, bc_cmb=b[0], bc_surface=b[1]).apply(u, path="slow")
         assert rel_err(out.cpu().numpy(), ref) < 1e-12
+
+
+@pytest.mark.parametrize("lat,rad", [(1, 2), (2, 2), (2, 3), (3, 2)])
+@pytest.mark.parametrize("q0", [False, True])
+@pytest.mark.parametrize("interpolation", [0, 1])
+def test_fast_gca_build_equals_plain_build(cuda, lat, rad, q0, interpolation):
+    """The build over on-the-fly matrices, 32 coarse hexes a block, against the plain one on cell counts that do not fill
+    the last block and with one or several radial layers; the two round differently in the last bits (1e-13)."""
+    g = T.Shell(lat, rad, num_levels=2)
+    nl, nr = g.dims(1)
+    nlc, nrc = g.dims(0)
+    rng = np.random.default_rng(lat + 10 * rad)
+    shape = (10, nl - 1, nl - 1, nr - 1) if q0 else (10, nl, nl, nr)
+    coef = _t(np.exp(rng.uniform(-2.0, 2.0, shape)))
+    fine = T.EpsDivDiv(g, 1, **({"k_cell": coef} if q0 else {"k": coef}))
+    mats = []
+    for fast in (True, False):
+        coarse = T.EpsDivDiv(g, 0, k=_t(np.ones((10, nlc, nlc, nrc))))
+        T.gca_build(fine, coarse, interpolation=interpolation, tensor_cores=fast)
+        mats.append(coarse.local_matrices())
+    assert rel_err(mats[0], mats[1]) < 1e-13
