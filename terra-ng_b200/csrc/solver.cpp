@@ -6,6 +6,7 @@
 // device memory. FGMRES waits for the device once per iteration, to read the
 // new Hessenberg column for the Givens rotations and the convergence test
 // (the reference waits at every dot product).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <limits>
@@ -213,15 +214,10 @@ VelocityMultigrid::VelocityMultigrid(const Shell* sh, const EpsDivDivOp& fine, c
     ops64_[0]->packed_layout = true;
     ops64_[0]->ensure_baked(false, st);
     {
-        const DeviceLevel& L0   = sh->level(0);
-        const int          nmem = static_cast<int>(L0.host.dup_members.size());
-        chk(coarse_pcg_prepare(L0.nl(), L0.nr(), L0.iface.num_classes, nmem), "coarse CG configuration");
-        if (coarse_pcg_uses_full_matrices(L0.nl(), L0.nr(), L0.iface.num_classes, nmem)) {
-            const int nc0 = static_cast<int>(L0.cells());
-            cfull_.alloc(sizeof(double) * 2 * 324 * static_cast<size_t>(nc0));
-            chk(coarse_matrices_unpack(nc0, ops64_[0]->baked64.as<double>(), cfull_.as<double>(), st), "unpack");
-            cuda_check(cudaStreamSynchronize(st), "unpack");
-        }
+        const DeviceLevel& L0 = sh->level(0);
+        chk(coarse_pcg_prepare(L0.nl(), L0.nr()), "coarse CG configuration");
+        const std::vector<int32_t> uid = number_coarse();
+        if (!o.coarse_dense) build_coarse_rows(uid, st);
     }
 
     if (o.coarse_dense) build_dense_coarse(st);
@@ -311,16 +307,14 @@ VelocityMultigrid::VelocityMultigrid(const Shell* sh, const EpsDivDivOp& fine, c
     cuda_check(cudaMemset(cstats_.get(), 0, sizeof(double) * 4), "zero stats");
 }
 
-// Dense inverse of the coarsest operator (coarse_dense.cu): unique-node numbering from the ownership flags and
-// the duplicate classes, one column per unknown from the stored operator applied to a unit vector that is 1 on
-// every copy of the unknown, then in-place Gauss-Jordan inversion. Synchronous set-up.
-void VelocityMultigrid::build_dense_coarse(cudaStream_t st)
+// Unique nodes of the coarsest level, numbered over the owned copies in storage order.
+std::vector<int32_t> VelocityMultigrid::number_coarse()
 {
-    const DeviceLevel& L0 = sh_->level(0);
-    const ShellLevel&  h  = L0.host;
-    const int          nr = L0.nr();
-    const int64_t      nodes = L0.nodes();
-    const int          nlat  = static_cast<int>(h.owned_lat.size());
+    const DeviceLevel&   L0    = sh_->level(0);
+    const ShellLevel&    h     = L0.host;
+    const int            nr    = L0.nr();
+    const int64_t        nodes = L0.nodes();
+    const int            nlat  = static_cast<int>(h.owned_lat.size());
     std::vector<int32_t> owner(nlat);
     for (int c = 0; c < nlat; ++c) owner[c] = c;
     for (size_t k = 0; k + 1 < h.dup_offset.size(); ++k) {
@@ -338,15 +332,85 @@ void VelocityMultigrid::build_dense_coarse(cudaStream_t st)
                 rep.push_back(static_cast<int32_t>(c * nr + r));
             }
     for (int c = 0; c < nlat; ++c)
-        for (int r = 0; r < nr; ++r) uid[static_cast<size_t>(c) * nr + r] = uid_owned[static_cast<size_t>(owner[c]) * nr + r];
-    knu_         = static_cast<int>(rep.size());
+        for (int r = 0; r < nr; ++r)
+            uid[static_cast<size_t>(c) * nr + r] = uid_owned[static_cast<size_t>(owner[c]) * nr + r];
+    knu_  = static_cast<int>(rep.size());
+    kuid_ = upload(uid);
+    krep_ = upload(rep);
+    return uid;
+}
+
+// Assembled rows of the coarsest operator (boundary conditions baked in) for coarse_cg_rows: the wedge matrices summed
+// over all cells around each unique node. Synchronous set-up.
+void VelocityMultigrid::build_coarse_rows(const std::vector<int32_t>& uid, cudaStream_t st)
+{
+    const DeviceLevel& L0 = sh_->level(0);
+    const int          nl = L0.nl(), nr = L0.nr(), nc = static_cast<int>(L0.cells());
+    if (!coarse_cg_rows_fit(knu_, 21)) return;  // 7 lateral x 3 radial neighbours
+    std::vector<double> mats(static_cast<size_t>(342) * nc);
+    cuda_check(cudaMemcpyAsync(mats.data(), ops64_[0]->baked64.get(), mats.size() * sizeof(double), cudaMemcpyDeviceToHost,
+                               st),
+               "copy matrices");
+    cuda_check(cudaStreamSynchronize(st), "copy matrices");
+    static constexpr int off[2][6][3] = {{{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {1, 0, 1}, {0, 1, 1}},
+                                         {{1, 1, 0}, {0, 1, 0}, {1, 0, 0}, {1, 1, 1}, {0, 1, 1}, {1, 0, 1}}};
+    std::vector<std::vector<int32_t>> nbr(knu_);
+    std::vector<std::vector<double>>  val(knu_);
+    int                               cell = 0;
+    for (int d = 0; d < 10; ++d)
+        for (int x = 0; x < nl - 1; ++x)
+            for (int y = 0; y < nl - 1; ++y)
+                for (int r = 0; r < nr - 1; ++r, ++cell)
+                    for (int w = 0; w < 2; ++w) {
+                        int32_t u[6];
+                        for (int n = 0; n < 6; ++n)
+                            u[n] = uid[static_cast<size_t>(((d * nl + x + off[w][n][0]) * nl + y + off[w][n][1])) * nr + r +
+                                       off[w][n][2]];
+                        for (int i = 0; i < 6; ++i)
+                            for (int j = 0; j < 6; ++j) {
+                                auto&  list = nbr[u[i]];
+                                size_t k    = 0;
+                                while (k < list.size() && list[k] != u[j]) ++k;
+                                if (k == list.size()) {
+                                    list.push_back(u[j]);
+                                    val[u[i]].resize(9 * list.size(), 0.0);
+                                }
+                                double* v = val[u[i]].data() + 9 * k;
+                                for (int a = 0; a < 3; ++a)
+                                    for (int b = 0; b < 3; ++b) {
+                                        const int p = std::min(i + 6 * a, j + 6 * b), q = std::max(i + 6 * a, j + 6 * b);
+                                        v[3 * a + b] +=
+                                            mats[static_cast<size_t>(w * 171 + p * (37 - p) / 2 + (q - p)) * nc + cell];
+                                    }
+                            }
+                    }
+    size_t m = 0;
+    for (const auto& l : nbr) m = std::max(m, l.size());
+    if (m > 21) return;
+    std::vector<int32_t> list(m * knu_, 0);
+    std::vector<double>  rows(9 * m * knu_, 0.0);
+    for (int u = 0; u < knu_; ++u) {
+        std::copy(nbr[u].begin(), nbr[u].end(), list.begin() + m * u);
+        std::copy(val[u].begin(), val[u].end(), rows.begin() + 9 * m * u);
+    }
+    if (!coarse_cg_rows_fit(knu_, static_cast<int>(m))) return;
+    cneighbours_ = static_cast<int>(m);
+    cnbr_        = upload(list);
+    crows_       = upload(rows);
+}
+
+// Dense inverse of the coarsest operator (coarse_dense.cu): unique-node numbering from the ownership flags and
+// the duplicate classes, one column per unknown from the stored operator applied to a unit vector that is 1 on
+// every copy of the unknown, then in-place Gauss-Jordan inversion. Synchronous set-up.
+void VelocityMultigrid::build_dense_coarse(cudaStream_t st)
+{
+    const DeviceLevel& L0    = sh_->level(0);
+    const int64_t      nodes = L0.nodes();
     const int nd = 3 * knu_;
     if (nd > kDenseCoarseMaxUnknowns)
         throw Error(kErrUnsupported, "the coarsest level is too large for the dense coarse solve (" +
                                          std::to_string(nd) + " unknowns)");
     chk(dense_coarse_prepare(nd), "dense coarse configuration");
-    kuid_ = upload(uid);
-    krep_ = upload(rep);
     ky_.alloc(sizeof(double) * nd);
     kinv_.alloc(sizeof(double) * static_cast<size_t>(nd) * nd);
     DevBuf        colk(sizeof(double) * nd);
@@ -535,15 +599,34 @@ void VelocityMultigrid::coarse_solve(T* x, const T* b, cudaStream_t st)
             chk(convert_f64_to_f32(nt, cx_.data(), reinterpret_cast<float*>(x), st), "narrow");
         return;
     }
+    if (crows_.get() != nullptr) {
+        CoarseCgArgs a;
+        a.nodes      = knu_;
+        a.neighbours = cneighbours_;
+        a.nbr        = cnbr_.as<int32_t>();
+        a.values     = crows_.as<double>();
+        a.rep        = krep_.as<int32_t>();
+        a.uid        = kuid_.as<int32_t>();
+        a.n          = static_cast<int>(L0.nodes());
+        a.stride     = pad64(L0.nodes());
+        a.x          = xd;
+        a.b          = bd;
+        a.max_iter   = opt_.coarse_max_iter;
+        a.rtol       = opt_.coarse_rtol;
+        a.atol       = opt_.coarse_atol;
+        a.stats      = cstats_.as<double>();
+        chk(coarse_cg_rows(a, st), "coarse CG");
+        if (!std::is_same<T, double>::value)
+            chk(convert_f64_to_f32(nt, cx_.data(), reinterpret_cast<float*>(x), st), "narrow");
+        return;
+    }
     EpsDivDivOp& A0 = *ops64_[0];
     A0.ensure_baked(false, st);
     CoarsePcgArgs a;
     a.nl          = L0.nl();
     a.nr          = L0.nr();
     a.mats        = A0.baked64.as<double>();
-    a.mats_full   = cfull_.size() ? cfull_.as<double>() : nullptr;
     a.num_classes = L0.iface.num_classes;
-    a.num_members = static_cast<int>(L0.host.dup_members.size());
     a.off         = L0.iface.offset;
     a.mem         = L0.iface.members;
     a.owned       = L0.owned_lat.as<uint8_t>();

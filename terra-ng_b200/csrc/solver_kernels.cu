@@ -9,9 +9,9 @@
 // * The Chebyshev-Jacobi update d = alpha D^-1 (b - A x) + beta d, x += d in one
 //   pass (chebyshev.hpp:102-176 uses four BLAS-1 launches per step).
 // * The coarsest-grid CG (pcg.hpp:81-169, identity preconditioner) as a single
-//   thread-block-cluster kernel over stored element matrices: the CTAs of one
-//   cluster synchronise with the hardware cluster barrier, so the whole solve is
-//   one launch.
+//   thread-block-cluster kernel over assembled rows, or over stored element matrices
+//   on levels too large for that: the CTAs of one cluster synchronise with the
+//   hardware cluster barrier, so the whole solve is one launch.
 #include <cfloat>
 #include <map>
 #include <mutex>
@@ -642,279 +642,147 @@ __global__ void __launch_bounds__(kPcgThreads, 1) coarse_pcg_kernel(CoarsePcgArg
 }
 
 // ---------------------------------------------------------------------------
-// Coarsest CG with the vectors replicated in every CTA's shared memory (levels
-// with up to ~2000 nodes, e.g. level 2). Each CTA applies its cells' matrices
-// to its local copy of p into a local partial (shared-memory atomics); the
-// partials are summed slice by slice over distributed shared memory and the
-// sums broadcast back, so after two cluster barriers every CTA holds the full
-// A p. Dots and vector updates then run on local copies, identically (same
-// data, same order) in every CTA, and need no further communication.
+// Coarsest CG over assembled rows (levels of up to a few thousand nodes, e.g. level 2). The unknowns are the unique
+// nodes, so there are no interface sums and no ownership masks; CTA k of the cluster owns a slice of them, with their
+// rows as 3 x 3 blocks over at most m neighbours in shared memory (77 KB a CTA at level 2), and every CTA keeps full
+// copies of p and r. An iteration is A p on the own rows (16 lanes a node), the cluster-wide <A p, p>, the own part of
+// r sent to all CTAs together with its <r, r>, and p = r + beta p on the full copies: two cluster barriers, both sums in
+// rank order, no atomics.
+//
+// Bound by latency (barriers and reductions). With element matrices, partial vectors summed over distributed shared
+// memory and interface sums, an iteration took 14.5 us at level 2.
 // ---------------------------------------------------------------------------
-// Block-wide sum returned to every thread. The warp sums go to one of two
-// buffers in turn, so a single barrier suffices: a buffer is written again
-// only two calls later, after every thread has passed the barrier of the call
-// in between (and so has finished reading it).
-__device__ double block_sum_all(double v, double* red, int& parity)
+constexpr int kRowLanes = 16;
+
+__device__ double cg_cluster_sum(double v, double* red, double* buf, cg::cluster_group& cluster)
 {
-    v           = warp_sum(v);
-    double* buf = red + (parity & 1) * 32;
-    ++parity;
-    if ((threadIdx.x & 31) == 0) buf[threadIdx.x >> 5] = v;
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
-    // every warp folds the warp sums with the same butterfly, so all threads
-    // (and all CTAs holding the same data) get identical bits
-    const int lane = threadIdx.x & 31;
-    return warp_sum(lane < static_cast<int>(blockDim.x >> 5) ? buf[lane] : 0.0);
-}
-
-// Owned-entry dot over the three components (own: one byte per entry of a
-// component, 1 where the lateral node is owned).
-__device__ __forceinline__ double owned_dot(const double* a, const double* b, int n, const uint8_t* own, double* red,
-                                             int& parity)
-{
-    double acc = 0.0;
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-        for (int j = threadIdx.x; j < n; j += blockDim.x)
-            if (own[j]) acc += a[c * n + j] * b[c * n + j];
-    return block_sum_all(acc, red, parity);
-}
-
-// Shared-memory tables of the replicated coarsest CG, built once per launch
-// (the work assignment does not change between iterations).
-struct RepTables {
-    const int32_t* node;     // [12][cpc]: node index of wedge node (w, n) of local cell lc
-    const uint8_t* own;      // [n]
-    const int32_t* mv_code;  // [items]: lc | (w * 18 + a) << 16
-    const int32_t* if_base;  // [iitems]: c * n + r of interface item
-    const int32_t* if_cls;   // [iitems]
-    const int32_t* cls_off;  // [num_classes + 1]
-    const int32_t* mem_nr;   // [members]: member lateral index * nr
-    int            items, iitems, cpc, c0;
-};
-
-// dst = A src (all CTAs end with the same full vector). part must be zero on
-// entry and is zero again on return. xch: blockDim.x doubles of scratch.
-// Each matvec item is one row a of one wedge's 18 x 18 matrix for one local
-// cell, read from the row-major copy mats_full[(w * 18 + a) * 18 + b][cell].
-__device__ void rep_matvec(const CoarsePcgArgs& A, const RepTables& R, const double* src, double* dst, double* part,
-                           double* xch, int n, int n3, int nc, cg::cluster_group& cluster)
-{
-    for (int k = 0; k < 2; ++k) {
-        const int it = threadIdx.x + k * blockDim.x;
-        if (it >= R.items) break;
-        const int      code = R.mv_code[it];
-        const int      lc = code & 0xffff, wa = code >> 16;
-        const int      w = wa >= 18 ? 1 : 0, a = wa - 18 * w;
-        const double*  row  = A.mats_full + static_cast<int64_t>(wa) * 18 * nc + (R.c0 + lc);
-        const int32_t* nd   = R.node + w * 6 * R.cpc + lc;
-        int            idx[6];
-#pragma unroll
-        for (int nb = 0; nb < 6; ++nb) idx[nb] = nd[nb * R.cpc];
-        double acc = 0.0;
-#pragma unroll
-        for (int b = 0; b < 18; ++b) acc += __ldg(row + static_cast<int64_t>(b) * nc) * src[(b / 6) * n + idx[b % 6]];
-        atomicAdd(part + (a / 6) * n + idx[a % 6], acc);
+    const unsigned ncta = cluster.num_blocks();
+    if (threadIdx.x < 32) {
+        const double s = warp_sum(red[threadIdx.x]);
+        if (threadIdx.x < ncta) cluster.map_shared_rank(buf, threadIdx.x)[cluster.block_rank()] = s;
     }
     cluster.sync();
-    // This CTA sums slice [e0, e1) over all CTAs' partials: thread t reads
-    // element e0 + t % sl from the CTAs k, k + ng, ... (k = t / sl), the ng
-    // group sums are combined in a fixed order, and the same thread layout
-    // writes the result to every CTA's dst.
-    const unsigned ncta = cluster.num_blocks(), rank = cluster.block_rank();
-    const int      sl   = (n3 + static_cast<int>(ncta) - 1) / static_cast<int>(ncta);
-    const int      e0 = static_cast<int>(rank) * sl, e1 = e0 + sl < n3 ? e0 + sl : n3;
-    const int      len = e1 > e0 ? e1 - e0 : 0;
-    if (sl <= static_cast<int>(blockDim.x)) {
-        int ng = static_cast<int>(blockDim.x) / sl;
-        if (ng > static_cast<int>(ncta)) ng = static_cast<int>(ncta);
-        const int t = threadIdx.x, k = t / sl, i = t - k * sl;
-        if (k < ng) {
-            double v = 0.0;
-            if (i < len)
-                for (int c = k; c < static_cast<int>(ncta); c += ng) v += cluster.map_shared_rank(part, c)[e0 + i];
-            xch[t] = v;
-        }
-        __syncthreads();
-        if (t < len) {  // column t: group sums in order k = 0, 1, ...
-            double v = xch[t];
-            for (int g = 1; g < ng; ++g) v += xch[g * sl + t];
-            xch[t] = v;
-        }
-        __syncthreads();
-        if (k < ng && i < len)
-            for (int c = k; c < static_cast<int>(ncta); c += ng) cluster.map_shared_rank(dst, c)[e0 + i] = xch[i];
-    } else {
-        for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-            double v = 0.0;
-            for (unsigned c = 0; c < ncta; ++c) v += cluster.map_shared_rank(part, c)[e];
-            for (unsigned c = 0; c < ncta; ++c) cluster.map_shared_rank(dst, c)[e] = v;
-        }
-    }
-    cluster.sync();
-    for (int e = threadIdx.x; e < n3; e += blockDim.x) part[e] = 0.0;
-    // interface sums: every copy of an interface node gets the class sum
-    for (int it = threadIdx.x; it < R.iitems; it += blockDim.x) {
-        double*   v  = dst + R.if_base[it];
-        const int cl = R.if_cls[it];
-        const int b0 = R.cls_off[cl], b1 = R.cls_off[cl + 1];
-        double    s  = 0.0;
-        for (int m = b0; m < b1; ++m) s += v[R.mem_nr[m]];
-        for (int m = b0; m < b1; ++m) v[R.mem_nr[m]] = s;
-    }
-    __syncthreads();
+    double s = 0.0;
+    for (unsigned k = 0; k < ncta; ++k) s += buf[k];
+    return s;
 }
 
-__global__ void __launch_bounds__(kPcgThreads, 1) coarse_pcg_rep_kernel(CoarsePcgArgs A)
+__global__ void __launch_bounds__(kPcgThreads, 1) coarse_cg_rows_kernel(CoarseCgArgs A)
 {
     extern __shared__ __align__(16) unsigned char pcg_smem[];
-    __shared__ double   red[2 * 32];
-    __shared__ double   xch[kPcgThreads];
-    int                 parity  = 0;
-    cg::cluster_group   cluster = cg::this_cluster();
-    const unsigned      rank = cluster.block_rank(), ncta = cluster.num_blocks();
-    const int           nl = A.nl, nr = A.nr;
-    const int           nc = 10 * (nl - 1) * (nl - 1) * (nr - 1);
-    const int           n = static_cast<int>(A.n), n3 = 3 * n;
-    const int64_t       S = A.stride;
-    const uint64_t      rdiv = reciprocal_nr(nr);
+    __shared__ double red[32];
+    __shared__ double sums[2][kPcgMaxCta];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = static_cast<int>(cluster.block_rank()), ncta = static_cast<int>(cluster.num_blocks());
+    const int nu = A.nodes, m = A.neighbours, npc = (nu + ncta - 1) / ncta;
+    const int u0 = rank * npc, cnt = max(min(npc, nu - u0), 0);
+    double*   p   = reinterpret_cast<double*>(pcg_smem);  // [node][3], full
+    double*   r   = p + 3 * nu;                           // full
+    double*   x   = r + 3 * nu;                           // own
+    double*   ap  = x + 3 * npc;                          // own
+    double*   val = ap + 3 * npc;                         // own rows [node][m][3][3]
+    int32_t*  nbr = reinterpret_cast<int32_t*>(A.rows_in_smem ? val + 9 * static_cast<size_t>(m) * npc : val);
 
-    // shared layout (offsets as in pcg_config): 4 vectors, node table, item
-    // codes, interface tables, ownership bytes
-    double*  p_s  = reinterpret_cast<double*>(pcg_smem);
-    double*  r_s  = p_s + n3;
-    double*  ap_s = r_s + n3;
-    double*  pt_s = ap_s + n3;
-    int32_t* node = reinterpret_cast<int32_t*>(pt_s + n3);
-    const int cpc = A.cells_per_cta;
-    int32_t*  mv_code = node + 12 * cpc;
-    const int items   = 36 * cpc;
-    const int iitems  = A.num_classes * nr * 3;
-    int32_t*  if_base = mv_code + items;
-    int32_t*  if_cls  = if_base + iitems;
-    int32_t*  cls_off = if_cls + iitems;
-    const int nmem    = A.num_classes > 0 ? A.off[A.num_classes] : 0;
-    int32_t*  mem_nr  = cls_off + A.num_classes + 1;
-    uint8_t*  own     = reinterpret_cast<uint8_t*>(mem_nr + nmem);
-
-    RepTables R;
-    R.cpc = cpc;
-    R.c0  = static_cast<int>(rank) * cpc;
-    int cnt = nc - R.c0 < cpc ? nc - R.c0 : cpc;
-    if (cnt < 0) cnt = 0;
-    R.items  = 36 * cnt;
-    R.iitems = iitems;
-    for (int i = threadIdx.x; i < 12 * cpc; i += blockDim.x) {
-        const int lc = i % cpc, k = i / cpc;
-        int32_t   v  = 0;
-        if (lc < cnt) {
-            const int cell = R.c0 + lc;
-            const int r    = cell % (nr - 1);
-            int       t    = cell / (nr - 1);
-            const int y    = t % (nl - 1);
-            t /= (nl - 1);
-            const int x = t % (nl - 1), d = t / (nl - 1);
-            const int w = k / 6, nn = k % 6;
-            v = static_cast<int32_t>(
-                node_index(nl, nr, d, x + woff_c(w, nn, 0), y + woff_c(w, nn, 1), r + woff_c(w, nn, 2)));
-        }
-        node[i] = v;
+    for (int i = threadIdx.x; i < 3 * nu; i += blockDim.x) p[i] = A.x[(i % 3) * A.stride + A.rep[i / 3]];
+    for (int i = threadIdx.x; i < 3 * cnt; i += blockDim.x) x[i] = A.x[(i % 3) * A.stride + A.rep[u0 + i / 3]];
+    for (int i = threadIdx.x; i < m * cnt; i += blockDim.x) nbr[i] = A.nbr[static_cast<int64_t>(u0) * m + i];
+    const double* rows = A.values + static_cast<int64_t>(u0) * m * 9;
+    if (A.rows_in_smem) {
+        for (int i = threadIdx.x; i < 9 * m * cnt; i += blockDim.x) val[i] = rows[i];
+        rows = val;
     }
-    for (int it = threadIdx.x; it < R.items; it += blockDim.x) {
-        const int lc = it % cnt, wa = it / cnt;  // wa = w * 18 + a
-        mv_code[it]  = lc | (wa << 16);
-    }
-    for (int it = threadIdx.x; it < iitems; it += blockDim.x) {
-        const int r = it % nr, rest = it / nr, c = rest % 3, cl = rest / 3;
-        if_base[it] = c * n + r;
-        if_cls[it]  = cl;
-    }
-    for (int i = threadIdx.x; i <= A.num_classes; i += blockDim.x) cls_off[i] = A.off[i];
-    for (int m = threadIdx.x; m < nmem; m += blockDim.x) mem_nr[m] = A.mem[m] * nr;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) own[j] = A.owned[lat_of(j, rdiv)] ? 1 : 0;
-    R.node    = node;
-    R.own     = own;
-    R.mv_code = mv_code;
-    R.if_base = if_base;
-    R.if_cls  = if_cls;
-    R.cls_off = cls_off;
-    R.mem_nr  = mem_nr;
-
-    // slice of x this CTA updates: at most one entry per thread
-    const int sl = (n3 + static_cast<int>(ncta) - 1) / static_cast<int>(ncta);
-    const int x0 = static_cast<int>(rank) * sl, x1 = x0 + sl < n3 ? x0 + sl : n3;
-    int       xe = -1;
-    int64_t   xg = 0;
-    if (x0 + static_cast<int>(threadIdx.x) < x1) {
-        xe          = x0 + threadIdx.x;
-        const int c = xe / n, j = xe - c * n;
-        xg          = c * S + j;
-    }
-
-    // r = b - A x, p = r
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-        for (int j = threadIdx.x; j < n; j += blockDim.x) {
-            p_s[c * n + j]  = A.x[c * S + j];
-            pt_s[c * n + j] = 0.0;
-        }
     __syncthreads();
-    rep_matvec(A, R, p_s, ap_s, pt_s, xch, n, n3, nc, cluster);
+
+    const int lane = threadIdx.x & (kRowLanes - 1), group = threadIdx.x / kRowLanes, groups = kPcgThreads / kRowLanes;
+    // ap = A p on the own rows; returns this thread's part of <A p, p>
+    auto product = [&]() {
+        double dot = 0.0;
+        for (int first = group & ~1; first < cnt; first += groups) {  // both halves of a warp make the same trips
+            const int u  = first + (group & 1);
+            double    y0 = 0.0, y1 = 0.0, y2 = 0.0;
+            if (u < cnt)
+                for (int k = lane; k < m; k += kRowLanes) {
+                    const double* v  = rows + (static_cast<int64_t>(u) * m + k) * 9;
+                    const double* q  = p + 3 * nbr[u * m + k];
+                    const double  q0 = q[0], q1 = q[1], q2 = q[2];
+                    y0 = fma(v[2], q2, fma(v[1], q1, fma(v[0], q0, y0)));
+                    y1 = fma(v[5], q2, fma(v[4], q1, fma(v[3], q0, y1)));
+                    y2 = fma(v[8], q2, fma(v[7], q1, fma(v[6], q0, y2)));
+                }
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
-        for (int j = threadIdx.x; j < n; j += blockDim.x) {
-            const double rv = A.b[c * S + j] - ap_s[c * n + j];
-            r_s[c * n + j]  = rv;
-            p_s[c * n + j]  = rv;
+            for (int o = kRowLanes / 2; o > 0; o >>= 1) {
+                y0 += __shfl_xor_sync(0xffffffffu, y0, o);
+                y1 += __shfl_xor_sync(0xffffffffu, y1, o);
+                y2 += __shfl_xor_sync(0xffffffffu, y2, o);
+            }
+            if (lane < 3 && u < cnt) {
+                const double y = lane == 0 ? y0 : (lane == 1 ? y1 : y2);
+                ap[3 * u + lane] = y;
+                dot += y * p[3 * (u0 + u) + lane];
+            }
         }
-    __syncthreads();
-    double       rr   = owned_dot(r_s, r_s, n, own, red, parity);
+        __syncthreads();
+        return dot;
+    };
+    // own part of r to every CTA
+    auto send_r = [&](int i, double v) {
+        for (int k = 0; k < ncta; ++k) cluster.map_shared_rank(r, k)[3 * u0 + i] = v;
+    };
+
+    (void)product();
+    cluster.sync();  // every CTA has started: its shared memory may be written
+    double acc = 0.0;
+    for (int i = threadIdx.x; i < 3 * cnt; i += blockDim.x) {
+        const double v = A.b[(i % 3) * A.stride + A.rep[u0 + i / 3]] - ap[i];
+        acc += v * v;
+        send_r(i, v);
+    }
+    double       rr   = cg_cluster_sum(acc, red, sums[1], cluster);
     const double init = sqrt(rr);
     double       res  = init;
     int          its  = 0;
+    for (int i = threadIdx.x; i < 3 * nu; i += blockDim.x) p[i] = r[i];
+    __syncthreads();
     if (!(init < A.atol)) {
         double an = rr;
         for (int it = 1; it <= A.max_iter; ++it) {
-            rep_matvec(A, R, p_s, ap_s, pt_s, xch, n, n3, nc, cluster);
-            const double ad = owned_dot(ap_s, p_s, n, own, red, parity);
+            const double ad = cg_cluster_sum(product(), red, sums[0], cluster);
             if (fabs(ad) < DBL_MIN) break;
             const double alpha = an / ad;
-            if (xe >= 0) A.x[xg] += alpha * p_s[xe];
-            for (int e = threadIdx.x; e < n3; e += blockDim.x) r_s[e] = r_s[e] - alpha * ap_s[e];
-            __syncthreads();
-            rr  = owned_dot(r_s, r_s, n, own, red, parity);
+            acc                = 0.0;
+            for (int i = threadIdx.x; i < 3 * cnt; i += blockDim.x) {
+                x[i] += alpha * p[3 * u0 + i];
+                const double v = r[3 * u0 + i] - alpha * ap[i];
+                acc += v * v;
+                send_r(i, v);
+            }
+            rr  = cg_cluster_sum(acc, red, sums[1], cluster);
             res = sqrt(rr);
             its = it;
             if (res / init <= A.rtol || res < A.atol) break;
             const double bn = rr;
             if (fabs(an) < DBL_MIN) break;
             const double beta = bn / an;
-            for (int e = threadIdx.x; e < n3; e += blockDim.x) p_s[e] = r_s[e] + beta * p_s[e];
+            for (int i = threadIdx.x; i < 3 * nu; i += blockDim.x) p[i] = r[i] + beta * p[i];
             __syncthreads();
             an = bn;
         }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < A.n; i += blockDim.x) {  // every copy of the own nodes
+        const int u = A.uid[i] - u0;
+        if (u >= 0 && u < cnt)
+            for (int c = 0; c < 3; ++c) A.x[c * A.stride + i] = x[3 * u + c];
     }
     if (rank == 0 && threadIdx.x == 0 && A.stats) {
         A.stats[0] = static_cast<double>(its);
         A.stats[1] = init;
         A.stats[2] = res;
     }
-    // no CTA may leave while others still read its shared memory
-    cluster.sync();
-}
-
-// Row-major copy of packed symmetric wedge matrices:
-// full[(w * 18 + a) * 18 + b][cell] = packed[w * 171 + pidx(a, b)][cell].
-__global__ void unpack_full_kernel(int nc, const double* __restrict__ packed, double* __restrict__ full)
-{
-    const int64_t total = static_cast<int64_t>(2) * 324 * nc;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        const int cell = static_cast<int>(i % nc);
-        const int rab  = static_cast<int>(i / nc);
-        const int w = rab / 324, ab = rab % 324, a = ab / 18, b = ab % 18;
-        full[i]     = packed[static_cast<int64_t>(w * 171 + pidx_rt(a, b)) * nc + cell];
-    }
+    cluster.sync();  // no CTA may leave while others still write to it
 }
 
 __global__ void inject_kernel(int nlc, int nrc, const double* __restrict__ fine, double* __restrict__ coarse,
@@ -1110,11 +978,10 @@ int widen_check(int64_t n, const float* in, double* out, int* flag_dev, cudaStre
 }
 
 namespace {
-using PcgKernel = void (*)(CoarsePcgArgs);
-
 // cluster size (16 when the device allows non-portable clusters of this
 // kernel with the given shared memory, else 8)
-int pcg_cluster_size(PcgKernel kernel, size_t smem)
+template <typename K>
+int pcg_cluster_size(K kernel, size_t smem)
 {
     int size = 8;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
@@ -1137,99 +1004,91 @@ int pcg_cluster_size(PcgKernel kernel, size_t smem)
     return size;
 }
 
+constexpr size_t kPcgSmemLimit = 200 * 1024;
+
+// Launch configuration of a coarsest level, decided once per level size and device (function attributes and
+// occupancy queries stay out of launches, so the launch can be captured in a graph).
 struct PcgConfig {
-    int       cs = 0, cpc = 0, in_smem = 0;
-    size_t    node_bytes = 0, smem = 0;
-    PcgKernel kernel = nullptr;
+    int    cs = 0, cpc = 0, in_smem = 0;
+    size_t node_bytes = 0, smem = 0;
 };
 
-// Launch configuration for a coarsest level (nodes per component n, nc
-// cells), decided once per level size (function attributes and occupancy
-// queries stay out of launches, so the launch can be captured in a graph).
-// Levels whose four vectors fit in shared memory run the replicated kernel.
-int pcg_config(int n, int nc, int nr, int ncls, int nmem, PcgConfig& out)
+int pcg_config(int nc, PcgConfig& out)
 {
-    static std::mutex                                           mu;
-    // per device: the function attributes set below belong to the current device
-    static std::map<std::tuple<int, int, int, int, int, int>, PcgConfig> cache;
-    std::lock_guard<std::mutex>                                      lock(mu);
-    int                                                              dev = 0;
+    static std::mutex                               mu;
+    static std::map<std::pair<int, int>, PcgConfig> cache;
+    std::lock_guard<std::mutex>                     lock(mu);
+    int                                             dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -2;
-    const auto key = std::make_tuple(dev, n, nc, nr, ncls, nmem);
-    auto                                                        it  = cache.find(key);
+    const auto key = std::make_pair(dev, nc);
+    auto       it  = cache.find(key);
     if (it != cache.end()) {
         out = it->second;
         return 0;
     }
-    constexpr size_t kSmemLimit = 200 * 1024;
-    PcgConfig        c;
-    const size_t     vec_bytes = static_cast<size_t>(4) * 3 * n * sizeof(double);
-    auto             layout    = [&](int cs) {
+    PcgConfig c;
+    auto      layout = [&](int cs) {
         c.cs         = cs;
         c.cpc        = (nc + cs - 1) / cs;
         c.node_bytes = (static_cast<size_t>(48) * c.cpc + 15) / 16 * 16;
-        // replicated kernel tables: item codes, interface items (base, class),
-        // class offsets, member indices, ownership bytes
-        const size_t iitems = static_cast<size_t>(ncls) * nr * 3;
-        const size_t tables = sizeof(int32_t) * (36 * static_cast<size_t>(c.cpc) + 2 * iitems + ncls + 1 + nmem) + n;
-        const size_t rep    = vec_bytes + c.node_bytes + (tables + 15) / 16 * 16;
-        if (rep <= kSmemLimit && 36 * c.cpc <= 2 * kPcgThreads) {
-            c.kernel  = coarse_pcg_rep_kernel;
-            c.smem    = rep;
-            c.in_smem = 0;
-        } else {
-            c.kernel  = coarse_pcg_kernel;
-            c.smem    = c.node_bytes + static_cast<size_t>(342 * 8) * c.cpc;
-            c.in_smem = c.smem <= kSmemLimit ? 1 : 0;
-            if (!c.in_smem) c.smem = c.node_bytes;
-        }
+        c.smem       = c.node_bytes + static_cast<size_t>(342 * 8) * c.cpc;
+        c.in_smem    = c.smem <= kPcgSmemLimit ? 1 : 0;
+        if (!c.in_smem) c.smem = c.node_bytes;
     };
     layout(kPcgMaxCta);
-    for (PcgKernel k : {static_cast<PcgKernel>(coarse_pcg_kernel), static_cast<PcgKernel>(coarse_pcg_rep_kernel)})
-        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemLimit)) !=
-            cudaSuccess) {
-            cudaGetLastError();
-            return -2;
-        }
-    if (pcg_cluster_size(c.kernel, c.smem) != kPcgMaxCta) layout(8);
-    if (c.node_bytes > kSmemLimit) return -1;
+    if (cudaFuncSetAttribute(coarse_pcg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(kPcgSmemLimit)) != cudaSuccess) {
+        cudaGetLastError();
+        return -2;
+    }
+    if (pcg_cluster_size(coarse_pcg_kernel, c.smem) != kPcgMaxCta) layout(8);
+    if (c.node_bytes > kPcgSmemLimit) return -1;
     cache[key] = c;
     out        = c;
     return 0;
 }
-}  // namespace
 
-int coarse_pcg_prepare(int nl, int nr, int num_classes, int num_members)
+// The same for the row kernel: cluster size, bytes, rows in shared memory or read from L2. cs = 0 where not even the
+// vectors fit.
+int rows_config(int nodes, int neighbours, PcgConfig& out)
 {
-    PcgConfig c;
-    return pcg_config(10 * nl * nl * nr, 10 * (nl - 1) * (nl - 1) * (nr - 1), nr, num_classes, num_members, c);
-}
-
-int coarse_pcg_uses_full_matrices(int nl, int nr, int num_classes, int num_members)
-{
-    PcgConfig c;
-    if (pcg_config(10 * nl * nl * nr, 10 * (nl - 1) * (nl - 1) * (nr - 1), nr, num_classes, num_members, c) != 0)
+    static std::mutex                                    mu;
+    static std::map<std::tuple<int, int, int>, PcgConfig> cache;
+    std::lock_guard<std::mutex>                          lock(mu);
+    int                                                  dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return -2;
+    const auto key = std::make_tuple(dev, nodes, neighbours);
+    auto       it  = cache.find(key);
+    if (it != cache.end()) {
+        out = it->second;
         return 0;
-    return c.kernel == coarse_pcg_rep_kernel ? 1 : 0;
+    }
+    PcgConfig c;
+    auto      layout = [&](int cs) {
+        const size_t npc  = static_cast<size_t>((nodes + cs - 1) / cs);
+        const size_t vecs = sizeof(double) * (6 * static_cast<size_t>(nodes) + 6 * npc), list = sizeof(int32_t) * npc * neighbours;
+        const size_t rows = sizeof(double) * 9 * npc * neighbours;
+        c.in_smem         = vecs + list + rows <= kPcgSmemLimit ? 1 : 0;
+        c.smem            = vecs + list + (c.in_smem ? rows : 0);
+        c.cs              = c.smem <= kPcgSmemLimit ? cs : 0;
+    };
+    layout(kPcgMaxCta);
+    if (c.cs != 0) {
+        if (cudaFuncSetAttribute(coarse_cg_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(kPcgSmemLimit)) != cudaSuccess) {
+            cudaGetLastError();
+            return -2;
+        }
+        if (pcg_cluster_size(coarse_cg_rows_kernel, c.smem) != kPcgMaxCta) layout(8);
+    }
+    cache[key] = c;
+    out        = c;
+    return 0;
 }
 
-int coarse_matrices_unpack(int nc, const double* packed, double* full, cudaStream_t st)
+template <typename K, typename Args>
+int launch_cluster(K kernel, const Args& args, const PcgConfig& c, cudaStream_t st)
 {
-    unpack_full_kernel<<<1184, 256, 0, st>>>(nc, packed, full);
-    return launch_status();
-}
-
-int coarse_pcg(const CoarsePcgArgs& args_in, cudaStream_t st)
-{
-    CoarsePcgArgs args = args_in;
-    const int     nc   = 10 * (args.nl - 1) * (args.nl - 1) * (args.nr - 1);
-    PcgConfig     c;
-    const int     rc = pcg_config(static_cast<int>(args.n), nc, args.nr, args.num_classes, args.num_members, c);
-    if (rc != 0) return rc;
-    if (c.kernel == coarse_pcg_rep_kernel && args.mats_full == nullptr) return -1;
-    args.cells_per_cta = c.cpc;
-    args.node_bytes    = static_cast<int>(c.node_bytes);
-    args.mats_in_smem  = c.in_smem;
     cudaLaunchConfig_t  cfg = {};
     cudaLaunchAttribute at[1];
     at[0].id               = cudaLaunchAttributeClusterDimension;
@@ -1243,11 +1102,47 @@ int coarse_pcg(const CoarsePcgArgs& args_in, cudaStream_t st)
     cfg.attrs              = at;
     cfg.numAttrs           = 1;
     note_launch();
-    if (cudaLaunchKernelEx(&cfg, c.kernel, args) != cudaSuccess) {
+    if (cudaLaunchKernelEx(&cfg, kernel, args) != cudaSuccess) {
         cudaGetLastError();
         return -2;
     }
     return 0;
+}
+}  // namespace
+
+int coarse_pcg_prepare(int nl, int nr)
+{
+    PcgConfig c;
+    return pcg_config(10 * (nl - 1) * (nl - 1) * (nr - 1), c);
+}
+
+int coarse_pcg(const CoarsePcgArgs& args_in, cudaStream_t st)
+{
+    CoarsePcgArgs args = args_in;
+    PcgConfig     c;
+    const int     rc = pcg_config(10 * (args.nl - 1) * (args.nl - 1) * (args.nr - 1), c);
+    if (rc != 0) return rc;
+    args.cells_per_cta = c.cpc;
+    args.node_bytes    = static_cast<int>(c.node_bytes);
+    args.mats_in_smem  = c.in_smem;
+    return launch_cluster(coarse_pcg_kernel, args, c, st);
+}
+
+bool coarse_cg_rows_fit(int nodes, int neighbours)
+{
+    PcgConfig c;
+    return rows_config(nodes, neighbours, c) == 0 && c.cs != 0;
+}
+
+int coarse_cg_rows(const CoarseCgArgs& args_in, cudaStream_t st)
+{
+    CoarseCgArgs args = args_in;
+    PcgConfig    c;
+    const int    rc = rows_config(args.nodes, args.neighbours, c);
+    if (rc != 0) return rc;
+    if (c.cs == 0) return -1;
+    args.rows_in_smem = c.in_smem;
+    return launch_cluster(coarse_cg_rows_kernel, args, c, st);
 }
 
 int coarse_pcg_partials_size() { return 2 * kPcgMaxCta; }

@@ -295,9 +295,7 @@ struct AxpyList {
 struct CoarsePcgArgs {
     int            nl = 0, nr = 0;
     const double*  mats        = nullptr;  // baked stored matrices of the level
-    const double*  mats_full   = nullptr;  // row-major copy (coarse_matrices_unpack), for the replicated kernel
     int            num_classes = 0;
-    int            num_members = 0;  // off[num_classes]
     const int32_t* off = nullptr;
     const int32_t* mem = nullptr;
     const uint8_t* owned = nullptr;
@@ -314,6 +312,26 @@ struct CoarsePcgArgs {
     // set by coarse_pcg: cells per CTA, bytes of the node table, matrices in shared memory
     int cells_per_cta = 0, node_bytes = 0, mats_in_smem = 0;
 };
+// Coarsest CG over assembled rows: unique nodes with their rows as 3 x 3 blocks over `neighbours` nodes (padded with
+// zero blocks); rep: stored index of a node's owned copy, uid: node of every stored copy.
+struct CoarseCgArgs {
+    int            nodes = 0, neighbours = 0;
+    const int32_t* nbr    = nullptr;  // [node][neighbours]
+    const double*  values = nullptr;  // [node][neighbours][3][3]
+    const int32_t* rep    = nullptr;
+    const int32_t* uid    = nullptr;
+    int            n      = 0;  // stored nodes
+    int64_t        stride = 0;  // component stride of x, b
+    double*        x      = nullptr;  // in: initial guess (equal on copies), out: solution on every copy
+    const double*  b      = nullptr;
+    int            max_iter = 50;
+    double         rtol = 1e-6, atol = 1e-16;
+    double*        stats = nullptr;  // as CoarsePcgArgs
+    int            rows_in_smem = 0;  // set by coarse_cg_rows
+};
+// also fixes the launch configuration (call before any stream capture); false where the vectors exceed shared memory
+bool coarse_cg_rows_fit(int nodes, int neighbours);
+int  coarse_cg_rows(const CoarseCgArgs& args, cudaStream_t st);
 int solver_partials_size();
 template <typename T>
 int vec_dot(const VecDesc& L, const T* a, const T* b, double* out_dev, RedScratch rs, bool take_sqrt, cudaStream_t st);
@@ -359,12 +377,7 @@ int flag_nonfinite(int64_t n, const T* a, int* flag_dev, cudaStream_t st);
 int widen_check(int64_t n, const float* in, double* out, int* flag_dev, cudaStream_t st);
 int coarse_pcg(const CoarsePcgArgs& args, cudaStream_t st);
 // decide and cache the launch configuration for a level (call outside graph capture)
-int coarse_pcg_prepare(int nl, int nr, int num_classes, int num_members);
-// 1 when the coarsest CG of this level runs the replicated kernel, which reads
-// the row-major matrix copy made by coarse_matrices_unpack
-int coarse_pcg_uses_full_matrices(int nl, int nr, int num_classes, int num_members);
-// full[(w * 18 + a) * 18 + b][cell] = packed[w * 171 + pidx(a, b)][cell], nc cells
-int coarse_matrices_unpack(int nc, const double* packed, double* full, cudaStream_t st);
+int coarse_pcg_prepare(int nl, int nr);
 int coarse_pcg_partials_size();
 
 // Dense direct coarsest solve (coarse_dense.cu). Unknown (c, u) = c * nu + u; uid maps every stored node to

@@ -96,6 +96,8 @@ class VelocityMultigrid {
     void vcycle(int l, T* x, const T* b, cudaStream_t st, bool x_zero);
     template <typename T>
     void coarse_solve(T* x, const T* b, cudaStream_t st);
+    std::vector<int32_t> number_coarse();      // knu_, krep_, kuid_; returns uid
+    void build_coarse_rows(const std::vector<int32_t>& uid, cudaStream_t st);  // crows_, where they fit
     void build_dense_coarse(cudaStream_t st);  // kinv_ = inverse of the assembled coarsest operator
 
     const Shell*                              sh_;
@@ -109,9 +111,11 @@ class VelocityMultigrid {
     Work<float>                               w32_;
     DVec<double>                              cx_, cb_, cr_, cp_, cap_;  // coarsest CG vectors
     DevBuf                                    cpart_, cstats_;
-    DevBuf                                    cfull_;  // row-major coarsest matrices (replicated CG)
-    DevBuf                                    kinv_, kuid_, krep_, ky_;  // dense coarsest solve
-    int                                       knu_ = 0;                  // unique coarsest nodes
+    DevBuf                                    crows_, cnbr_;  // assembled coarsest rows (coarse_cg_rows)
+    int                                       cneighbours_ = 0;
+    DevBuf                                    kinv_, ky_;    // dense coarsest solve
+    DevBuf                                    kuid_, krep_;  // unique coarsest nodes (number_coarse)
+    int                                       knu_ = 0;
     DVec<double>                              ext64_[2];
     DVec<float>                               ext32_[2];
 };

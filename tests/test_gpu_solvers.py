@@ -589,3 +589,27 @@ def test_fast_gca_build_equals_plain_build(cuda, lat, rad, q0, interpolation):
         T.gca_build(fine, coarse, interpolation=interpolation, tensor_cores=fast)
         mats.append(coarse.local_matrices())
     assert rel_err(mats[0], mats[1]) < 1e-13
+
+
+@pytest.mark.parametrize("lat,rad,nlev", [(1, 2, 2), (2, 2, 2), (3, 3, 3), (3, 4, 2), (4, 4, 2)])
+def test_coarse_cg_equals_dense_solve(cuda, lat, rad, nlev):
+    """The coarsest CG run to convergence against the dense solve, on coarsest levels of a few nodes a CTA (and CTAs
+    without any), with rows in shared memory, and too large for the row kernel: the V-cycles agree to the CG's 1e-13
+    times the conditioning of the level (1e-9, as against the oracle)."""
+    import torch
+
+    g = T.Shell(lat, rad, num_levels=nlev)
+    nl, nr = g.dims(nlev - 1)
+    sh = O.Shell(lat, rad)
+    k = smooth_viscosity(sh, 29, 100.0)
+    b = O.enforce_rhs_bcs(sh, consistent(sh, O.seeded_normal(sh.vec_shape, 30)), 1, 2)
+    res = []
+    for kw in ({"coarse_solver": T.COARSE_DENSE}, {"coarse_relative_tolerance": 1e-13, "coarse_max_iterations": 4000}):
+        try:
+            s = T.VelocitySolver(g, eta=_t(k), bc_cmb=1, bc_surface=2, **kw)
+        except T.TerraError:  # the dense solve has a size limit
+            pytest.skip("coarsest level too large for the dense solve")
+        x = torch.zeros(sh.vec_shape, dtype=torch.float64, device=cuda)
+        s.vcycle(x, _t(b))
+        res.append(x.cpu().numpy())
+    assert rel_err(res[1], res[0]) < 1e-9
