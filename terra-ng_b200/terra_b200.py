@@ -200,6 +200,22 @@ def _comps(v):
     return [v]
 
 
+_POINTERS = [ctypes.c_void_p * n for n in range(5)]
+
+
+def _pointers(v):
+    """Component addresses of a vector (a list of component tensors, a (ncomp, ...) tensor, or one scalar field),
+    without making a tensor per component: slicing the six of one operator apply took longer than the apply itself on
+    the small levels."""
+    if isinstance(v, (list, tuple)):
+        return _ptrs(v)
+    base = v.data_ptr()
+    if v.dim() != 5:
+        return _POINTERS[1](base)
+    n, step = v.shape[0], v.stride(0) * v.element_size()
+    return (_POINTERS[n] if n < 5 else ctypes.c_void_p * n)(*[base + c * step for c in range(n)])
+
+
 def _stream(stream):
     if stream is None:
         import torch
@@ -353,10 +369,12 @@ class Operator:
         _check(load().tn_operator_set_boundary_conditions(self._h, bc_cmb, bc_surface))
 
     def apply(self, src, dst, stream=None):
-        cs, cd = _comps(src), _comps(dst)
-        if len(cs) != self.src_components or len(cd) != self.dst_components:
+        ps, pd = _pointers(src), _pointers(dst)
+        if len(ps) != self.src_components or len(pd) != self.dst_components:
             raise ValueError(f"operator takes {self.src_components} -> {self.dst_components} components")
-        _check(load().tn_operator_apply(self._h, _ptrs(cs), _ptrs(cd), _stream(stream)))
+        rc = _lib.tn_operator_apply(self._h, ps, pd, _stream(stream))
+        if rc != TN_OK:
+            _check(rc)
         return dst
 
 
