@@ -604,12 +604,12 @@ int tn_restrict(tn_shell* shell, int fine_level, int precision, int ncomp, const
         int         rc;
         if (precision == TN_F64) {
             auto c = reinterpret_cast<double* const*>(coarse_dev);
-            rc     = tn::restrict_owned<double>(L.nl(), L.nr(), ncomp, L.owned_lat.as<uint8_t>(),
+            rc     = tn::restrict_owned<double>(L.nl(), L.nr(), ncomp, L.owned_lat.as<uint8_t>(), nullptr,
                                             reinterpret_cast<const double* const*>(fine_dev), c, as_stream(stream));
             if (!rc) rc = tn::interface_sum<double>(Lc.iface, Lc.nr(), ncomp, c, as_stream(stream));
         } else {
             auto c = reinterpret_cast<float* const*>(coarse_dev);
-            rc     = tn::restrict_owned<float>(L.nl(), L.nr(), ncomp, L.owned_lat.as<uint8_t>(),
+            rc     = tn::restrict_owned<float>(L.nl(), L.nr(), ncomp, L.owned_lat.as<uint8_t>(), nullptr,
                                            reinterpret_cast<const float* const*>(fine_dev), c, as_stream(stream));
             if (!rc) rc = tn::interface_sum<float>(Lc.iface, Lc.nr(), ncomp, c, as_stream(stream));
         }

@@ -550,19 +550,21 @@ void VelocityMultigrid::vcycle(int l, T* x, const T* b, cudaStream_t st, bool x_
     smooth<T>(l, x, b, st, x_zero);
     T* res = W.tmp[l].data();
     apply<T>(l, x, res, st);
-    const T one_m[2] = {T(1), T(-1)};
-    lin<T>(W.tmp[l].total(), res, T(0), 2, one_m, b, res, st);
     const int64_t sf = pad64(L.nodes()), sc = pad64(Lc.nodes());
     T*            rc = W.r[l - 1].data();
     T*            ec = W.e[l - 1].data();
     const T*      fin[3]  = {res, res + sf, res + 2 * sf};
+    const T*      bin[3]  = {b, b + sf, b + 2 * sf};
     T*            cout[3] = {rc, rc + sc, rc + 2 * sc};
-    if (opt_.transfer == 1)
+    if (opt_.transfer == 1) {
+        const T one_m[2] = {T(1), T(-1)};
+        lin<T>(W.tmp[l].total(), res, T(0), 2, one_m, b, res, st);
         chk(restrict_linear_owned<T>(L.nl(), L.nr(), 3, L.owned_lat.as<uint8_t>(), L.linear_weights<T>(st), fin,
                                      cout, st),
             "restrict");
-    else
-        chk(restrict_owned<T>(L.nl(), L.nr(), 3, L.owned_lat.as<uint8_t>(), fin, cout, st), "restrict");
+    } else {
+        chk(restrict_owned<T>(L.nl(), L.nr(), 3, L.owned_lat.as<uint8_t>(), bin, fin, cout, st), "restrict");
+    }
     chk(interface_sum<T>(Lc.iface, Lc.nr(), 3, cout, st), "interface sum");
     cuda_check(cudaMemsetAsync(ec, 0, sizeof(T) * W.e[l - 1].total(), st), "zero correction");
     vcycle<T>(l - 1, ec, rc, st, true);

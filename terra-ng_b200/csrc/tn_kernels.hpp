@@ -117,12 +117,13 @@ int vector_mass_add(int nl, int nr, const T* coords, const T* radii, const T* co
 // prolongate_add: fine += P coarse (gather per fine node).
 // restrict_owned: coarse = sum over owned fine neighbours (weights of
 //                 prolongation_constant_weight); the interface sum follows.
+//                 With b, of b - fine in place of fine (the residual's restriction).
 // ----------------------------------------------------------------------------
 template <typename T>
 int prolongate_add(int nlf, int nrf, int ncomp, const T* const* coarse, T* const* fine, cudaStream_t stream);
 template <typename T>
-int restrict_owned(int nlf, int nrf, int ncomp, const uint8_t* owned_lat_fine, const T* const* fine, T* const* coarse,
-                   cudaStream_t stream);
+int restrict_owned(int nlf, int nrf, int ncomp, const uint8_t* owned_lat_fine, const T* const* b, const T* const* fine,
+                   T* const* coarse, cudaStream_t stream);
 
 // Linear transfers (transfer_linear.cu): w holds two weights per fine node (linear_transfer_weights, FP64
 // from the fine coordinates; FP32 copies for the FP32 V-cycle).
