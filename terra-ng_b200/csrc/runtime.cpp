@@ -124,7 +124,12 @@ const float* DeviceLevel::linear_weights<float>(cudaStream_t st) const
 template <typename T>
 void zero_components(int64_t n, int ncomp, T* const* v, cudaStream_t st)
 {
-    for (int c = 0; c < ncomp; ++c) cuda_check(cudaMemsetAsync(v[c], 0, static_cast<size_t>(n) * sizeof(T), st), "zero");
+    for (int c = 0; c < ncomp;) {  // adjacent components in one call
+        int e = c + 1;
+        while (e < ncomp && v[e] == v[e - 1] + n) ++e;
+        cuda_check(cudaMemsetAsync(v[c], 0, static_cast<size_t>(n) * (e - c) * sizeof(T), st), "zero");
+        c = e;
+    }
 }
 template void zero_components<double>(int64_t, int, double* const*, cudaStream_t);
 template void zero_components<float>(int64_t, int, float* const*, cudaStream_t);
@@ -458,7 +463,7 @@ template void EpsDivDivOp::vjp_logeta<double>(const double* const*, const double
 template void EpsDivDivOp::vjp_logeta<float>(const float* const*, const float* const*, float*, cudaStream_t) const;
 
 template <typename T>
-void EpsDivDivOp::apply_t(const T* const* src, T* const* dst, cudaStream_t st)
+void EpsDivDivOp::apply_t(const T* const* src, T* const* dst, cudaStream_t st, bool dst_zero)
 {
     const DeviceLevel& L = lvl();
     for (int c = 0; c < 3; ++c) {
@@ -466,7 +471,7 @@ void EpsDivDivOp::apply_t(const T* const* src, T* const* dst, cudaStream_t st)
         check_aligned<T>(dst[c]);
     }
     if (stored) {
-        if (apply_mode == 0) zero_components<T>(L.nodes(), 3, dst, st);
+        if (apply_mode == 0 && !dst_zero) zero_components<T>(L.nodes(), 3, dst, st);
         if (diagonal) {
             if (!std::is_same<T, double>::value)
                 throw Error(kErrUnsupported, "diagonal mode of a stored operator is FP64 only");
@@ -536,8 +541,8 @@ void EpsDivDivOp::apply_t(const T* const* src, T* const* dst, cudaStream_t st)
     add_penalty<T>(src, dst, st);
     if (comm_mode == 1) iface<T>(L, 3, dst, st);
 }
-template void EpsDivDivOp::apply_t<double>(const double* const*, double* const*, cudaStream_t);
-template void EpsDivDivOp::apply_t<float>(const float* const*, float* const*, cudaStream_t);
+template void EpsDivDivOp::apply_t<double>(const double* const*, double* const*, cudaStream_t, bool);
+template void EpsDivDivOp::apply_t<float>(const float* const*, float* const*, cudaStream_t, bool);
 
 void EpsDivDivOp::apply(void* const* src, void* const* dst, cudaStream_t st)
 {

@@ -472,31 +472,40 @@ double VelocityMultigrid::power_iteration(int l, int iterations, uint64_t seed, 
 }
 
 template <typename T>
-void VelocityMultigrid::apply(int l, const T* x, T* y, cudaStream_t st)
+bool VelocityMultigrid::adds(int l) const
+{
+    return (std::is_same<T, float>::value && ops32_[l] ? ops32_[l] : ops64_[l])->stored;
+}
+
+// With y_zero the caller knows y to hold zeros, which saves a stored operator clearing it.
+template <typename T>
+void VelocityMultigrid::apply(int l, const T* x, T* y, cudaStream_t st, bool y_zero)
 {
     const DeviceLevel& L = sh_->level(l);
     const int64_t      s = pad64(L.nodes());
     const T*           src[3] = {x, x + s, x + 2 * s};
     T*                 dst[3] = {y, y + s, y + 2 * s};
     if (std::is_same<T, float>::value && ops32_[l])
-        ops32_[l]->apply_t<T>(src, dst, st);
+        ops32_[l]->apply_t<T>(src, dst, st, y_zero);
     else
-        ops64_[l]->apply_t<T>(src, dst, st);
+        ops64_[l]->apply_t<T>(src, dst, st, y_zero);
 }
 
 // Chebyshev::solve_impl (chebyshev.hpp:102-176); rho carries over between the
 // outer iterations as in the reference. With x_zero (x holds zeros on entry,
 // as in every pre-smoothing of a V-cycle that starts from zero) the first
-// step's A x is exactly zero and is written as zeros instead of applied.
+// step's A x is exactly zero and is not applied; x is then written without being
+// read. Each update leaves the product vector zeroed where the level's operator
+// adds into it (`clear`), so only a first apply clears.
 template <typename T>
 void VelocityMultigrid::smooth(int l, T* x, const T* b, cudaStream_t st, bool x_zero)
 {
-    Work<T>& W = work<T>();
-    auto     residual_apply = [&](T* ax, bool first) {
-        if (first && x_zero)
+    Work<T>&   W     = work<T>();
+    const bool clear = adds<T>(l);
+    auto       residual_apply = [&](T* ax, bool first) {
+        if (first && !x_zero && clear)
             cuda_check(cudaMemsetAsync(ax, 0, sizeof(T) * W.tmp[l].total(), st), "zero");
-        else
-            apply<T>(l, x, ax, st);
+        if (!first || !x_zero) apply<T>(l, x, ax, st, clear);
     };
     if (opt_.smoother == 1) {
         // Jacobi::solve_impl (jacobi.hpp:51-60): x += omega D^-1 (b - A x), one
@@ -507,7 +516,9 @@ void VelocityMultigrid::smooth(int l, T* x, const T* b, cudaStream_t st, bool x_
         const T*      invd = W.invdiag[l].data();
         for (int it = 0; it < opt_.cheb_iters; ++it) {
             residual_apply(ax, it == 0);
-            chk(cheb_step<T>(n, x, d, b, ax, invd, static_cast<T>(opt_.jacobi_omega), T(0), true, st), "jacobi");
+            chk(cheb_step<T>(n, x, d, b, ax, invd, static_cast<T>(opt_.jacobi_omega), T(0), true, x_zero && it == 0,
+                             clear, st),
+                "jacobi");
         }
         return;
     }
@@ -523,13 +534,15 @@ void VelocityMultigrid::smooth(int l, T* x, const T* b, cudaStream_t st, bool x_
     const T*      invd  = W.invdiag[l].data();
     for (int it = 0; it < opt_.cheb_iters; ++it) {
         residual_apply(ax, it == 0);
-        chk(cheb_step<T>(n, x, d, b, ax, invd, static_cast<T>(1.0 / theta), T(0), true, st), "chebyshev");
+        chk(cheb_step<T>(n, x, d, b, ax, invd, static_cast<T>(1.0 / theta), T(0), true, x_zero && it == 0, clear,
+                         st),
+            "chebyshev");
         for (int i = 2; i <= opt_.cheb_order; ++i) {
             const double rho_new = 1.0 / (2.0 * sigma - rho);
             const double beta    = rho_new * rho;
             const double alpha   = 2.0 * rho_new / delta;
-            apply<T>(l, x, ax, st);
-            chk(cheb_step<T>(n, x, d, b, ax, invd, static_cast<T>(alpha), static_cast<T>(beta), false, st),
+            apply<T>(l, x, ax, st, clear);
+            chk(cheb_step<T>(n, x, d, b, ax, invd, static_cast<T>(alpha), static_cast<T>(beta), false, false, clear, st),
                 "chebyshev");
             rho = rho_new;
         }
@@ -549,7 +562,7 @@ void VelocityMultigrid::vcycle(int l, T* x, const T* b, cudaStream_t st, bool x_
     const DeviceLevel& Lc = sh_->level(l - 1);
     smooth<T>(l, x, b, st, x_zero);
     T* res = W.tmp[l].data();
-    apply<T>(l, x, res, st);
+    apply<T>(l, x, res, st, opt_.cheb_iters > 0 && adds<T>(l));  // zeroed by the smoother's last update
     const int64_t sf = pad64(L.nodes()), sc = pad64(Lc.nodes());
     T*            rc = W.r[l - 1].data();
     T*            ec = W.e[l - 1].data();
@@ -566,7 +579,8 @@ void VelocityMultigrid::vcycle(int l, T* x, const T* b, cudaStream_t st, bool x_
         chk(restrict_owned<T>(L.nl(), L.nr(), 3, L.owned_lat.as<uint8_t>(), bin, fin, cout, st), "restrict");
     }
     chk(interface_sum<T>(Lc.iface, Lc.nr(), 3, cout, st), "interface sum");
-    cuda_check(cudaMemsetAsync(ec, 0, sizeof(T) * W.e[l - 1].total(), st), "zero correction");
+    if (l == 1 || opt_.cheb_iters < 1)  // else the first smoothing step writes the correction without reading it
+        cuda_check(cudaMemsetAsync(ec, 0, sizeof(T) * W.e[l - 1].total(), st), "zero correction");
     vcycle<T>(l - 1, ec, rc, st, true);
     const T* cin[3]  = {ec, ec + sc, ec + 2 * sc};
     T*       fout[3] = {x, x + sf, x + 2 * sf};

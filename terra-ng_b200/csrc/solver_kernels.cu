@@ -338,16 +338,22 @@ __global__ void scale_recip_kernel(int64_t n, T* __restrict__ y, const T* __rest
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) y[i] = f * x[i];
 }
 
-template <typename T, bool FIRST>
+// Bound by memory on the large levels and by the launch on the small ones, so the kernel takes what would be launches and
+// passes of their own: FIRST starts a recurrence (d is not read), FROM_ZERO takes x = 0 and A x = 0 as known (neither is
+// read), CLEAR leaves ax zeroed for the stored operators, which add into their output. With three memsets an
+// apply, and a pass that wrote A x = 0, the level-6 mixed preconditioner took 3.52 ms instead of 3.16 and the level-4
+// velocity solve 18.8 ms instead of 16.5.
+template <typename T, bool FIRST, bool FROM_ZERO, bool CLEAR>
 __global__ void cheb_kernel(int64_t n, T* __restrict__ x, T* __restrict__ d, const T* __restrict__ b,
-                            const T* __restrict__ ax, const T* __restrict__ invd, T alpha, T beta)
+                            T* __restrict__ ax, const T* __restrict__ invd, T alpha, T beta)
 {
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const T z  = (b[i] - ax[i]) * invd[i];
+        const T z  = (FROM_ZERO ? b[i] : b[i] - ax[i]) * invd[i];
         const T dn = FIRST ? alpha * z : alpha * z + beta * d[i];
         d[i]       = dn;
-        x[i]       = x[i] + dn;
+        x[i]       = FROM_ZERO ? dn : x[i] + dn;
+        if (CLEAR) ax[i] = T(0);
     }
 }
 
@@ -918,18 +924,21 @@ template int scale_by_recip<double>(int64_t, double*, const double*, const doubl
 template int scale_by_recip<float>(int64_t, float*, const float*, const double*, cudaStream_t);
 
 template <typename T>
-int cheb_step(int64_t n, T* x, T* d, const T* b, const T* ax, const T* invdiag, T alpha, T beta, bool first,
-              cudaStream_t st)
+int cheb_step(int64_t n, T* x, T* d, const T* b, T* ax, const T* invdiag, T alpha, T beta, bool first, bool from_zero,
+              bool clear, cudaStream_t st)
 {
-    if (first)
-        cheb_kernel<T, true><<<grid_for(n), kThreads, 0, st>>>(n, x, d, b, ax, invdiag, alpha, beta);
+    const auto launch = [&](auto kernel) { kernel<<<grid_for(n), kThreads, 0, st>>>(n, x, d, b, ax, invdiag, alpha, beta); };
+    if (from_zero)
+        launch(clear ? cheb_kernel<T, true, true, true> : cheb_kernel<T, true, true, false>);
+    else if (first)
+        launch(clear ? cheb_kernel<T, true, false, true> : cheb_kernel<T, true, false, false>);
     else
-        cheb_kernel<T, false><<<grid_for(n), kThreads, 0, st>>>(n, x, d, b, ax, invdiag, alpha, beta);
+        launch(clear ? cheb_kernel<T, false, false, true> : cheb_kernel<T, false, false, false>);
     return launch_status();
 }
-template int cheb_step<double>(int64_t, double*, double*, const double*, const double*, const double*, double, double,
-                               bool, cudaStream_t);
-template int cheb_step<float>(int64_t, float*, float*, const float*, const float*, const float*, float, float, bool,
+template int cheb_step<double>(int64_t, double*, double*, const double*, double*, const double*, double, double, bool,
+                               bool, bool, cudaStream_t);
+template int cheb_step<float>(int64_t, float*, float*, const float*, float*, const float*, float, float, bool, bool, bool,
                               cudaStream_t);
 
 template <typename T>

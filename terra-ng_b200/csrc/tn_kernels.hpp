@@ -361,8 +361,8 @@ template <typename T>
 int scale_by_recip(int64_t n, T* y, const T* x, const double* s_dev, cudaStream_t st);
 // Chebyshev step: d = alpha D^-1 (b - ax) [+ beta d], x += d (flat)
 template <typename T>
-int cheb_step(int64_t n, T* x, T* d, const T* b, const T* ax, const T* invdiag, T alpha, T beta, bool first,
-              cudaStream_t st);
+int cheb_step(int64_t n, T* x, T* d, const T* b, T* ax, const T* invdiag, T alpha, T beta, bool first, bool from_zero,
+              bool clear, cudaStream_t stream);
 // y = c (a .* b) (flat)
 template <typename T>
 int vec_mul(int64_t n, T* y, const T* a, const T* b, T c, cudaStream_t st);

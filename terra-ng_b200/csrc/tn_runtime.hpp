@@ -277,7 +277,7 @@ struct EpsDivDivOp : Operator {
     int  dst_components() const override { return 3; }
     void apply(void* const* src, void* const* dst, cudaStream_t st) override;
     template <typename T>
-    void apply_t(const T* const* src, T* const* dst, cudaStream_t st);
+    void apply_t(const T* const* src, T* const* dst, cudaStream_t st, bool dst_zero = false);
     // backward of the apply: grad_cell = d(lambda^T A u)/d log(eta_cell) (Q0 only)
     template <typename T>
     void vjp_logeta(const T* const* u, const T* const* lam, T* grad_cell, cudaStream_t st) const;

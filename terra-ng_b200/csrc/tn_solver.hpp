@@ -89,7 +89,10 @@ class VelocityMultigrid {
     template <typename T>
     Work<T>& work();
     template <typename T>
-    void apply(int l, const T* x, T* y, cudaStream_t st);
+    void apply(int l, const T* x, T* y, cudaStream_t st, bool y_zero = false);
+    // the operator of level l adds into its output
+    template <typename T>
+    bool adds(int l) const;
     template <typename T>
     void smooth(int l, T* x, const T* b, cudaStream_t st, bool x_zero);
     template <typename T>
