@@ -390,6 +390,50 @@ def test_stokes_preconditioner_matches_oracle(cuda):
     assert rel_err(z[3].cpu().numpy(), zp) < 1e-12
 
 
+def test_preconditioner_large_level_precisions_agree(cuda):
+    """Level 6, where the smoother's update streams past L2: the mixed form against FP64. FP32 rounds to 6e-8 and the
+    V-cycle's contraction keeps its 60 updates from adding up; 4e-6 is some 60 roundings in one direction."""
+    import torch
+
+    sh = T.Shell(6, num_levels=5)
+    k = torch.exp(torch.tensor(O.Shell(6).coords[..., 0], device=cuda))[..., None].expand(10, 65, 65, 65).contiguous()
+    gen = torch.Generator(device=cuda).manual_seed(46)
+    nl, nr = sh.dims(-1)
+    u = [torch.randn((10, nl, nl, nr), dtype=torch.float64, device=cuda, generator=gen) for _ in range(3)]
+    for c in u:
+        sh.interface_sum(c)
+    v = u + [torch.zeros((10, 33, 33, 33), dtype=torch.float64, device=cuda)]
+    out = []
+    for mixed in (0, 1):
+        solver = T.StokesSolver(sh, eta=k, bc_cmb=1, bc_surface=1, chebyshev_order=3, coarse_solver=T.COARSE_DENSE,
+                                mixed_precision=mixed)
+        z = [torch.zeros_like(t) for t in v]
+        solver.precondition(v, z)
+        out.append(torch.stack(z[:3]))
+    assert torch.isfinite(out[1]).all()
+    assert ((out[1] - out[0]).norm() / out[0].norm()).item() < 4e-6
+
+
+def test_stored_apply_component_layouts(cuda):
+    """Adjacent output components are cleared in one call, others one by one; what lies between is left alone."""
+    import torch
+
+    g = T.Shell(3, num_levels=2)
+    ops = []
+    for l in (1, 2):
+        nl, nr = g.dims(-l)
+        ops.append(T.EpsDivDiv(g, -l, k=torch.ones((10, nl, nl, nr), dtype=torch.float64, device=cuda), bc_cmb=1, bc_surface=2))
+    T.gca_build(ops[0], ops[1])
+    src = torch.tensor(O.seeded_normal((3, 10, nl, nl, nr), 47), device=cuda)
+    one = torch.full_like(src, float("nan"))
+    ops[1].apply(src, one)
+    wide = torch.full((5, 10, nl, nl, nr), 7.0, dtype=torch.float64, device=cuda)
+    ops[1].apply(src, [wide[0], wide[1], wide[3]])
+    # the same sums of up to 72 atomic additions a node, in any order
+    assert rel_err(wide[[0, 1, 3]].cpu().numpy(), one.cpu().numpy()) < 1e-14
+    assert (wide[[2, 4]] == 7.0).all()
+
+
 def _max_duplicate_spread(g, level, v):
     """Largest difference between copies of one node (v: (ncomp, 10, nl, nl, nr))."""
     cls, n = g.duplicate_classes(level)
