@@ -206,6 +206,7 @@ __global__ void __launch_bounds__(Shape<T>::kThreads, 1) epsdivdiv_kernel(const 
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
+    chain_enter();
 
     // One barrier a row for the compute warps and the two staging warps. Barrier B(f) ends the cells of row f: the
     // exchange sums of row f are written, the reads of staged row f are done, row f + 2 has been treated.
@@ -808,7 +809,7 @@ int launch_cfg(const EddArgs<T>& a, size_t smem, int ctas, cudaStream_t st)
             configured[dev] = smem;
         }
     }
-    k<<<ctas, Shape<T>::kThreads, smem, st>>>(a);
+    launch_chained(k, ctas, Shape<T>::kThreads, smem, st, a);
     note_launch();
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

@@ -947,6 +947,7 @@ __device__ __forceinline__ void inner_matvec(const T* m, int64_t ni, const T (&s
 template <typename T, bool kStream>
 __global__ void __launch_bounds__(128, 3) gca_apply_compact_kernel(GcaApplyArgs<T> A, int inner_blocks)
 {
+    chain_enter();
     const int nl = A.nl, nr = A.nr, nrc = nr - 1, ncol = 10 * (nl - 1) * (nl - 1);
     const int ni = ncol * (nrc - 2), nb = 2 * ncol;
     int       d, x, y, r;
@@ -1261,9 +1262,9 @@ int gca_apply_compact_add(int nl, int nr, const T* mats, const T* const* src, T*
     const int  inner  = (2 * ncol * (nr - 3) + 127) / 128, edge = (4 * ncol + 127) / 128;
     const bool stream = gca_compact_values(nl, nr) * static_cast<int64_t>(sizeof(T)) > kGcaStreamBytes;
     if (stream)
-        gca_apply_compact_kernel<T, true><<<inner + edge, 128, 0, st>>>(a, inner);
+        launch_chained(gca_apply_compact_kernel<T, true>, inner + edge, 128, 0, st, a, inner);
     else
-        gca_apply_compact_kernel<T, false><<<inner + edge, 128, 0, st>>>(a, inner);
+        launch_chained(gca_apply_compact_kernel<T, false>, inner + edge, 128, 0, st, a, inner);
     return launch_status();
 }
 template int gca_apply_compact_add<double>(int, int, const double*, const double* const*, double* const*, cudaStream_t);

@@ -345,9 +345,9 @@ __global__ void scale_recip_kernel(int64_t n, T* __restrict__ y, const T* __rest
 // apply, and a pass that wrote A x = 0, the level-6 mixed preconditioner took 3.52 ms instead of 3.16 and the level-4
 // velocity solve 18.8 ms instead of 16.5.
 // STREAM: the vectors that only this kernel touches (b, d, D^-1) pass with evict-first, so that x and A x, which the
-// operator reads and writes around it, stay in L2. Taken where the
-// seven vectors outgrow half of L2: with 16-byte accesses the level-6 mixed preconditioner went from 3.16 to 2.97 ms, and
-// the level-4 velocity solve, whose vectors stay in L2, did not change.
+// operator reads and writes around it, stay in L2. Taken where the seven vectors outgrow half of L2: with 16-byte accesses
+// the level-6 mixed preconditioner went from 3.16 to 2.97 ms, and the level-4 velocity solve, whose vectors stay in L2, did
+// not change.
 template <typename T>
 struct alignas(16) Pack {
     T v[16 / sizeof(T)];
@@ -373,9 +373,9 @@ __device__ __forceinline__ void store_pack(T* p, const Pack<T>& r)
 }
 
 template <typename T, bool FIRST, bool FROM_ZERO, bool CLEAR, bool STREAM>
-__global__ void cheb_kernel(int64_t n, T* __restrict__ x, T* __restrict__ d, const T* __restrict__ b,
-                            T* __restrict__ ax, const T* __restrict__ invd, T alpha, T beta)
+__global__ void cheb_kernel(int64_t n, T* x, T* d, const T* b, T* ax, const T* invd, T alpha, T beta)
 {
+    chain_enter();
     constexpr int kV     = 16 / sizeof(T);  // n and the vectors are multiples of 64 elements
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x * kV;
     for (int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * kV; i < n; i += stride) {
@@ -969,7 +969,8 @@ int cheb_step(int64_t n, T* x, T* d, const T* b, T* ax, const T* invdiag, T alph
 {
     if (n % 64 != 0) return -1;
     const auto launch = [&](auto kernel) {
-        kernel<<<grid_for(n * static_cast<int64_t>(sizeof(T)) / 16), kThreads, 0, st>>>(n, x, d, b, ax, invdiag, alpha, beta);
+        launch_chained(kernel, grid_for(n * static_cast<int64_t>(sizeof(T)) / 16), kThreads, 0, st, n, x, d, b, ax, invdiag,
+                       alpha, beta);
     };
     const auto pick = [&](auto stream) {
         constexpr bool S = decltype(stream)::value;

@@ -96,6 +96,35 @@ __device__ __forceinline__ void report_error(int* err, int code)
     if (err) atomicCAS(err, 0, code);
 }
 
+// Chained launches (programmatic dependent launch). A kernel launched with launch_chained may start while the kernel
+// before it in its stream drains, so every thread of it calls chain_enter() before it touches memory that another kernel
+// writes: it waits until that kernel has completed and its writes are visible (and that kernel has waited for the one
+// before it), and then lets the next one start early. Such kernels read mutable memory through pointers without
+// __restrict__, so that no load counts as invariant and moves above the wait.
+// What it gives: about 1 to 2 us a launch, which is most of what the operators, sums and updates of the small levels take.
+// Level-4 velocity solve 15.8 -> 12.6 ms, level-6 mixed preconditioner 2.97 -> 2.64 ms, level-3 apply 14.1 -> 12.7 us.
+__device__ __forceinline__ void chain_enter()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute at[1];
+    at[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim            = grid;
+    cfg.blockDim           = block;
+    cfg.dynamicSmemBytes   = smem;
+    cfg.stream             = st;
+    cfg.attrs              = at;
+    cfg.numAttrs           = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 template <typename T>
 __device__ __forceinline__ T shfl_up(T v, int delta)
 {

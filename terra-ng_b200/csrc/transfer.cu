@@ -41,9 +41,10 @@ __global__ void __launch_bounds__(kTransferThreads) prolongate_kernel(int nlf, i
 {
     const int nlc = (nlf + 1) / 2, nrc = (nrf + 1) / 2;
     const int i   = blockIdx.x * blockDim.x + threadIdx.x;
+    chain_enter();
     if (i >= n) return;
-    const T* __restrict__ in  = P.in[blockIdx.y];
-    T* __restrict__       out = P.out[blockIdx.y];
+    const T* in  = P.in[blockIdx.y];
+    T*       out = P.out[blockIdx.y];
     int d, x, y, r, col;
     decode4(i, rad, lat, d, x, y, r, col);
     // lateral parents: one, or two across an edge (along x, along y, or the anti-diagonal), and radial parents
@@ -72,9 +73,10 @@ __global__ void __launch_bounds__(kTransferThreads) restrict_kernel(int nlf, int
                                                                     PtrSet<T> P, int n, Decoder rad, Decoder lat)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    chain_enter();
     if (i >= n) return;
-    const T* __restrict__ in = P.in[blockIdx.y];
-    const T* __restrict__ b  = RESIDUAL ? P.b[blockIdx.y] : nullptr;
+    const T* in = P.in[blockIdx.y];
+    const T* b  = RESIDUAL ? P.b[blockIdx.y] : nullptr;
     int d, xc, yc, rc, col;
     decode4(i, rad, lat, d, xc, yc, rc, col);
     // 7-point lateral stencil (prolongation_constant_fine_grid_stencil_offsets_at_coarse_vertex)
@@ -128,7 +130,7 @@ int prolongate_add(int nlf, int nrf, int ncomp, const T* const* coarse, T* const
     }
     const int n = 10 * nlf * nlf * nrf;
     const dim3 g((n + kTransferThreads - 1) / kTransferThreads, ncomp);
-    prolongate_kernel<T><<<g, kTransferThreads, 0, st>>>(nlf, nrf, P, n, Decoder(nrf), Decoder(nlf));
+    launch_chained(prolongate_kernel<T>, g, kTransferThreads, 0, st, nlf, nrf, P, n, Decoder(nrf), Decoder(nlf));
     return launch_status();
 }
 
@@ -147,9 +149,11 @@ int restrict_owned(int nlf, int nrf, int ncomp, const uint8_t* owned_lat_fine, c
     const int  n = 10 * nlc * nlc * nrc;
     const dim3 g((n + kTransferThreads - 1) / kTransferThreads, ncomp);
     if (b)
-        restrict_kernel<T, true><<<g, kTransferThreads, 0, st>>>(nlf, nrf, owned_lat_fine, P, n, Decoder(nrc), Decoder(nlc));
+        launch_chained(restrict_kernel<T, true>, g, kTransferThreads, 0, st, nlf, nrf, owned_lat_fine, P, n, Decoder(nrc),
+                       Decoder(nlc));
     else
-        restrict_kernel<T, false><<<g, kTransferThreads, 0, st>>>(nlf, nrf, owned_lat_fine, P, n, Decoder(nrc), Decoder(nlc));
+        launch_chained(restrict_kernel<T, false>, g, kTransferThreads, 0, st, nlf, nrf, owned_lat_fine, P, n, Decoder(nrc),
+                       Decoder(nlc));
     return launch_status();
 }
 

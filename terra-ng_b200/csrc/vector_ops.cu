@@ -37,9 +37,13 @@ __global__ void iface_kernel(int num_classes, const int32_t* __restrict__ off, c
     const int cls = blockIdx.x;
     const int c   = blockIdx.z;
     const int r   = blockIdx.y * blockDim.x + threadIdx.x;
-    if (cls >= num_classes || r >= nr || c >= ncomp) return;
+    if (cls >= num_classes || r >= nr || c >= ncomp) {
+        chain_enter();
+        return;
+    }
     const int b = __ldg(off + cls), e = __ldg(off + cls + 1);
     T*        p = v.p[c];
+    chain_enter();
     constexpr int kMax = 8;
     if (e - b <= kMax) {
         int64_t idx[kMax];
@@ -230,7 +234,7 @@ int interface_sum(const IfaceTable& t, int nr, int ncomp, T* const* comps, cudaS
     for (int c = 0; c < ncomp; ++c) v.p[c] = comps[c];
     const int threads = std::min(256, (nr + 31) / 32 * 32);
     dim3      grid(t.num_classes, (nr + threads - 1) / threads, ncomp);
-    iface_kernel<T><<<grid, threads, 0, stream>>>(t.num_classes, t.offset, t.members, nr, ncomp, v);
+    launch_chained(iface_kernel<T>, grid, threads, 0, stream, t.num_classes, t.offset, t.members, nr, ncomp, v);
     return launch_status();
 }
 
