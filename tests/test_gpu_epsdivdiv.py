@@ -208,3 +208,26 @@ def test_lateral_and_radial_levels(cuda, lat, rad, bcs):
             op.apply(src, part)
             op.apply(src, acc)
             assert rel_err(acc.double().cpu().numpy(), (src + part).double().cpu().numpy()) < tol
+
+
+@pytest.mark.parametrize("level", [2, 5])
+def test_chained_applies_equal_synchronised(cuda, level):
+    """Back-to-back launches overlap at their ends; a chain of dependent applies gives the bits of one that waits."""
+    import torch
+
+    g = T.Shell(level)
+    nl, nr = g.dims(-1)
+    A = T.EpsDivDiv(g, -1, k=torch.ones((10, nl, nl, nr), dtype=torch.float64, device=cuda), bc_cmb=1, bc_surface=2)
+    out = []
+    for wait in (False, True):
+        u = torch.tensor(O.seeded_normal((3, 10, nl, nl, nr), 48), device=cuda)
+        v = torch.empty_like(u)
+        torch.cuda.synchronize()
+        for _ in range(24):
+            A.apply(u, v)
+            if wait:
+                torch.cuda.synchronize()
+            u, v = v, u
+        torch.cuda.synchronize()
+        out.append(u)
+    assert torch.isfinite(out[0]).all() and torch.equal(out[0], out[1])
