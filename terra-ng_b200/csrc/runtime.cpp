@@ -425,6 +425,14 @@ void EpsDivDivOp::prepare_boundary(cudaStream_t st)
         (void)boundary_table<float>(k.as<float>(), st);
 }
 
+void EpsDivDivOp::prepare_apply(bool need32, cudaStream_t st)
+{
+    if (!stored) prepare_boundary(st);
+    if (stored || (selective && sel_built && sel_count > 0)) ensure_baked(need32, st);
+    prepare_penalty(st);
+    cuda_check(cudaStreamSynchronize(st), "prepare apply");
+}
+
 template <typename T>
 void EpsDivDivOp::add_penalty(const T* const* src, T* const* dst, cudaStream_t st)
 {

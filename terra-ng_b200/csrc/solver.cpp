@@ -291,6 +291,11 @@ VelocityMultigrid::VelocityMultigrid(const Shell* sh, const EpsDivDivOp& fine, c
     // lambda_max of D^-1 A per level for the Chebyshev smoother (the Jacobi smoother needs none)
     if (o.smoother == 0)
         for (int l = 1; l <= fine_; ++l) lambda_[l] = power_iteration(l, o.power_iters, o.seed + 7919ull * l, st);
+    // whatever the smoother and the precision, no later apply builds anything: Arnoldi steps are captured
+    for (int l = 1; l <= fine_; ++l) {
+        ops64_[l]->prepare_apply(o.fp32, st);
+        if (ops32_[l]) ops32_[l]->prepare_apply(false, st);
+    }
     // one FP32 apply per level now: kernel attributes are set outside any later graph capture
     if (o.fp32)
         for (int l = 1; l <= fine_; ++l) apply<float>(l, w32_.e[l].data(), w32_.tmp[l].data(), st);

@@ -286,6 +286,9 @@ struct EpsDivDivOp : Operator {
     template <typename T>
     const T* boundary_table(const T* kk, cudaStream_t st);
     void prepare_boundary(cudaStream_t st);  // the table of the operator's own precision
+    // everything a (non-diagonal) apply builds on first use, so that it can be captured (synchronous); need32: FP32
+    // applies of the stored matrices too
+    void prepare_apply(bool need32, cudaStream_t st);
     bool penalty_active() const { return bc_cmb == 2 && bc_surf == 2; }
     void prepare_penalty(cudaStream_t st);  // orthonormalises the modes (synchronous); no-op unless active or done
     template <typename T>

@@ -657,3 +657,33 @@ def test_coarse_cg_equals_dense_solve(cuda, lat, rad, nlev):
         s.vcycle(x, _t(b))
         res.append(x.cpu().numpy())
     assert rel_err(res[1], res[0]) < 1e-9
+
+
+@pytest.mark.parametrize("gca", [0, 1, 2])
+@pytest.mark.parametrize("nlev", [2, 3])
+@pytest.mark.parametrize("bcs,mixed", [((1, 2), 0), ((1, 2), 1), ((2, 2), 0)])
+def test_jacobi_solve_under_capture(cuda, gca, nlev, bcs, mixed):
+    """The captured Arnoldi steps with the Jacobi smoother, whose set-up applies no level's operator: every table an
+    apply needs is there before the capture. Same residual history as without graphs: with the dense coarsest solve a step
+    is one linear map, which two runs evaluate with atomic sums in another order (1e-16 in FP64 and 6e-8 in FP32 an
+    operation, a few hundred of them in sequence, times the conditioning), bounded here by 1e-9 and 1e-4 of the initial
+    residual. (The coarsest CG is no such map: stopped after 50 steps or at 1e-6, it passes rounding on at up to 1e-5.)
+    Free slip on both boundaries makes the coarsest level singular: CG there, and that it runs is what is tested."""
+    import torch
+
+    g = T.Shell(3, num_levels=nlev)
+    k = smooth_viscosity(O.Shell(3), 33, 1000.0)
+    f = T.stokes_rhs_enforce(g, -1, T.random_vector(g, nlev - 1, 3, 6), *bcs)
+    nl, nr = g.dims(-2)
+    b = [f[c].contiguous() for c in range(3)] + [torch.zeros((10, nl, nl, nr), dtype=torch.float64, device=cuda)]
+    hist = []
+    for graphs in (1, 0):
+        s = T.StokesSolver(g, eta=_t(k), bc_cmb=bcs[0], bc_surface=bcs[1], gca=gca, smoother=T.SMOOTHER_JACOBI,
+                           jacobi_omega=0.5, mixed_precision=mixed, cuda_graphs=graphs, max_iterations=8,
+                           coarse_solver=T.COARSE_PCG if bcs == (2, 2) else T.COARSE_DENSE,
+                           relative_tolerance=1e-14, absolute_tolerance=0.0)
+        s.solve([torch.zeros_like(t) for t in b], b)
+        hist.append(np.array(s.history()))
+    assert len(hist[0]) == len(hist[1]) > 8 and np.isfinite(hist[0]).all()
+    if bcs != (2, 2):
+        assert np.abs(hist[0] - hist[1]).max() < (1e-4 if mixed else 1e-9)
