@@ -803,13 +803,15 @@ __host__ __device__ constexpr int pair_col(int p)
 // (the level-4 FP32 matrices of a level-6 hierarchy, 56 MB).
 constexpr int64_t kGcaStreamBytes = 64ll << 20;
 
+// Neither form counts as invariant: the matrices of a chained kernel may have been rebuilt just before it, and no load
+// may move above its wait (chain_enter).
 template <typename T, bool kStream>
 __device__ __forceinline__ T ld_mat(const T* p)
 {
     if constexpr (kStream)
         return __ldcs(p);
     else
-        return __ldg(p);
+        return __ldca(p);
 }
 
 // o += A s over packed entries P.. with compile-time (row, column)
