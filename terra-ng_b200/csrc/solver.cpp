@@ -216,8 +216,8 @@ VelocityMultigrid::VelocityMultigrid(const Shell* sh, const EpsDivDivOp& fine, c
     {
         const DeviceLevel& L0 = sh->level(0);
         chk(coarse_pcg_prepare(L0.nl(), L0.nr()), "coarse CG configuration");
-        const std::vector<int32_t> uid = number_coarse();
-        if (!o.coarse_dense) build_coarse_rows(uid, st);
+        const std::vector<int32_t> owner = number_coarse();
+        if (!o.coarse_dense) build_coarse_rows(owner, st);
     }
 
     if (o.coarse_dense) build_dense_coarse(st);
@@ -342,66 +342,40 @@ std::vector<int32_t> VelocityMultigrid::number_coarse()
     knu_  = static_cast<int>(rep.size());
     kuid_ = upload(uid);
     krep_ = upload(rep);
-    return uid;
+    return owner;
 }
 
 // Assembled rows of the coarsest operator (boundary conditions baked in) for coarse_cg_rows: the wedge matrices summed
 // over all cells around each unique node. Synchronous set-up.
-void VelocityMultigrid::build_coarse_rows(const std::vector<int32_t>& uid, cudaStream_t st)
+void VelocityMultigrid::build_coarse_rows(const std::vector<int32_t>& owner, cudaStream_t st)
 {
     const DeviceLevel& L0 = sh_->level(0);
-    const int          nl = L0.nl(), nr = L0.nr(), nc = static_cast<int>(L0.cells());
-    if (!coarse_cg_rows_fit(knu_, 21)) return;  // 7 lateral x 3 radial neighbours
-    std::vector<double> mats(static_cast<size_t>(342) * nc);
-    cuda_check(cudaMemcpyAsync(mats.data(), ops64_[0]->baked64.get(), mats.size() * sizeof(double), cudaMemcpyDeviceToHost,
-                               st),
-               "copy matrices");
-    cuda_check(cudaStreamSynchronize(st), "copy matrices");
-    static constexpr int off[2][6][3] = {{{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {1, 0, 1}, {0, 1, 1}},
-                                         {{1, 1, 0}, {0, 1, 0}, {1, 0, 0}, {1, 1, 1}, {0, 1, 1}, {1, 0, 1}}};
-    std::vector<std::vector<int32_t>> nbr(knu_);
-    std::vector<std::vector<double>>  val(knu_);
-    int                               cell = 0;
-    for (int d = 0; d < 10; ++d)
-        for (int x = 0; x < nl - 1; ++x)
-            for (int y = 0; y < nl - 1; ++y)
-                for (int r = 0; r < nr - 1; ++r, ++cell)
-                    for (int w = 0; w < 2; ++w) {
-                        int32_t u[6];
-                        for (int n = 0; n < 6; ++n)
-                            u[n] = uid[static_cast<size_t>(((d * nl + x + off[w][n][0]) * nl + y + off[w][n][1])) * nr + r +
-                                       off[w][n][2]];
-                        for (int i = 0; i < 6; ++i)
-                            for (int j = 0; j < 6; ++j) {
-                                auto&  list = nbr[u[i]];
-                                size_t k    = 0;
-                                while (k < list.size() && list[k] != u[j]) ++k;
-                                if (k == list.size()) {
-                                    list.push_back(u[j]);
-                                    val[u[i]].resize(9 * list.size(), 0.0);
-                                }
-                                double* v = val[u[i]].data() + 9 * k;
-                                for (int a = 0; a < 3; ++a)
-                                    for (int b = 0; b < 3; ++b) {
-                                        const int p = std::min(i + 6 * a, j + 6 * b), q = std::max(i + 6 * a, j + 6 * b);
-                                        v[3 * a + b] +=
-                                            mats[static_cast<size_t>(w * 171 + p * (37 - p) / 2 + (q - p)) * nc + cell];
-                                    }
-                            }
-                    }
-    size_t m = 0;
-    for (const auto& l : nbr) m = std::max(m, l.size());
-    if (m > 21) return;
-    std::vector<int32_t> list(m * knu_, 0);
-    std::vector<double>  rows(9 * m * knu_, 0.0);
-    for (int u = 0; u < knu_; ++u) {
-        std::copy(nbr[u].begin(), nbr[u].end(), list.begin() + m * u);
-        std::copy(val[u].begin(), val[u].end(), rows.begin() + 9 * m * u);
-    }
-    if (!coarse_cg_rows_fit(knu_, static_cast<int>(m))) return;
-    cneighbours_ = static_cast<int>(m);
-    cnbr_        = upload(list);
-    crows_       = upload(rows);
+    const int          m  = coarse_cg_row_width(L0.nl(), L0.nr());
+    if (!coarse_cg_rows_fit(knu_, m)) return;
+    // copies of every owned lateral node, ascending, behind their offsets
+    const int            nlat = static_cast<int>(owner.size()), nown = knu_ / L0.nr();
+    std::vector<int32_t> number(nlat, -1), table(static_cast<size_t>(nown) + 1 + nlat, 0);
+    for (int c = 0, o = 0; c < nlat; ++c)
+        if (owner[c] == c) number[c] = o++;
+    for (int c = 0; c < nlat; ++c) ++table[number[owner[c]] + 1];
+    for (int o = 0; o < nown; ++o) table[o + 1] += table[o];
+    std::vector<int32_t> next(table.begin(), table.begin() + nown);
+    for (int c = 0; c < nlat; ++c) table[nown + 1 + next[number[owner[c]]]++] = c;
+    const DevBuf copies = upload(table);
+    DevBuf       nbr(sizeof(int32_t) * m * knu_), rows(sizeof(double) * 9 * m * knu_);
+    int          bad = 0;
+    DevBuf       flag(sizeof(int));
+    cuda_check(cudaMemsetAsync(flag.get(), 0, sizeof(int), st), "clear flag");
+    chk(coarse_cg_rows_assemble(L0.nl(), L0.nr(), knu_, m, ops64_[0]->baked64.as<double>(), copies.as<int32_t>(),
+                                copies.as<int32_t>() + nown + 1, kuid_.as<int32_t>(), nbr.as<int32_t>(),
+                                rows.as<double>(), flag.as<int>(), st),
+        "assemble rows");
+    cuda_check(cudaMemcpyAsync(&bad, flag.get(), sizeof(int), cudaMemcpyDeviceToHost, st), "copy flag");
+    cuda_check(cudaStreamSynchronize(st), "assemble rows");
+    if (bad) throw Error(kErrState, "a coarsest node with more neighbours than a regular mesh has");
+    cneighbours_ = m;
+    cnbr_        = std::move(nbr);
+    crows_       = std::move(rows);
 }
 
 // Dense inverse of the coarsest operator (coarse_dense.cu): unique-node numbering from the ownership flags and

@@ -332,6 +332,14 @@ struct CoarseCgArgs {
 };
 // also fixes the launch configuration (call before any stream capture); false where the vectors exceed shared memory
 bool coarse_cg_rows_fit(int nodes, int neighbours);
+// Neighbours of a node of the regular triangulation times the radial ones: the row width of a level.
+int coarse_cg_row_width(int nl, int nr);
+// Rows of a level from its baked packed matrices [342][cells]: nbr [node][m] and values [node][m][3][3] (zero blocks where
+// a row is shorter), m = coarse_cg_row_width. Node u = o nr + r for owned lateral node o; copies[copy_off[o] ..] are its
+// lateral copies, ascending; uid as in CoarseCgArgs. *flag = 1 where a row does not fit.
+int coarse_cg_rows_assemble(int nl, int nr, int nodes, int m, const double* mats, const int32_t* copy_off,
+                            const int32_t* copies, const int32_t* uid, int32_t* nbr, double* values, int* flag,
+                            cudaStream_t st);
 int  coarse_cg_rows(const CoarseCgArgs& args, cudaStream_t st);
 int solver_partials_size();
 template <typename T>

@@ -99,8 +99,8 @@ class VelocityMultigrid {
     void vcycle(int l, T* x, const T* b, cudaStream_t st, bool x_zero);
     template <typename T>
     void coarse_solve(T* x, const T* b, cudaStream_t st);
-    std::vector<int32_t> number_coarse();      // knu_, krep_, kuid_; returns uid
-    void build_coarse_rows(const std::vector<int32_t>& uid, cudaStream_t st);  // crows_, where they fit
+    std::vector<int32_t> number_coarse();  // knu_, krep_, kuid_; returns the owned copy of every lateral node
+    void build_coarse_rows(const std::vector<int32_t>& owner, cudaStream_t st);  // crows_, where they fit
     void build_dense_coarse(cudaStream_t st);  // kinv_ = inverse of the assembled coarsest operator
 
     const Shell*                              sh_;

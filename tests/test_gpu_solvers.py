@@ -635,7 +635,7 @@ def test_fast_gca_build_equals_plain_build(cuda, lat, rad, q0, interpolation):
     assert rel_err(mats[0], mats[1]) < 1e-13
 
 
-@pytest.mark.parametrize("lat,rad,nlev", [(1, 2, 2), (2, 2, 2), (3, 3, 3), (3, 4, 2), (4, 4, 2)])
+@pytest.mark.parametrize("lat,rad,nlev", [(1, 2, 2), (1, 3, 2), (2, 2, 2), (3, 2, 2), (3, 3, 2), (3, 3, 3), (3, 4, 2), (4, 4, 2)])
 def test_coarse_cg_equals_dense_solve(cuda, lat, rad, nlev):
     """The coarsest CG run to convergence against the dense solve, on coarsest levels of a few nodes a CTA (and CTAs
     without any), with rows in shared memory, and too large for the row kernel: the V-cycles agree to the CG's 1e-13
