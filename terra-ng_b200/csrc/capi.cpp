@@ -82,9 +82,8 @@ void init_edd(tn::EpsDivDivOp& e, tn::Shell* sh, int level, int precision, const
     e.bc_cmb    = bc_cmb;
     e.bc_surf   = bc_surface;
     e.diagonal  = diagonal != 0;
-    const size_t n = static_cast<size_t>(e.q0 ? L.cells() : L.nodes());
-    e.k.alloc(n * es);
-    tn::cuda_check(cudaMemcpy(e.k.get(), e.q0 ? k_cell_dev : k_nodal_dev, n * es, cudaMemcpyDeviceToDevice),
+    e.alloc_coefficient(e.k, es);
+    tn::cuda_check(cudaMemcpy(e.k.get(), e.q0 ? k_cell_dev : k_nodal_dev, e.k.size(), cudaMemcpyDeviceToDevice),
                    "copy coefficient");
     e.prepare_boundary(nullptr);
 }

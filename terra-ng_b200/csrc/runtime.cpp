@@ -271,12 +271,13 @@ void EpsDivDivOp::prepare_fp32(cudaStream_t st)
     if (precision != 0) return;
     if (selective && k32.get() == nullptr) {
         const int64_t n = static_cast<int64_t>(k.size() / sizeof(double));
-        DevBuf        b(sizeof(float) * static_cast<size_t>(n));
+        DevBuf        b;
+        alloc_coefficient(b, sizeof(float));
         if (convert_f64_to_f32(n, k.as<double>(), b.as<float>(), st) != 0)
             throw Error(kErrCuda, "conversion launch failed");
         k32 = std::move(b);
     }
-    if (selective) (void)boundary_table<float>(k32.as<float>(), st);
+    if (selective) (void)boundary_table<float>(st);
     prepare_penalty(st);
     cuda_check(cudaStreamSynchronize(st), "prepare fp32");
 }
@@ -397,32 +398,47 @@ void EpsDivDivOp::prepare_penalty(cudaStream_t st)
     pen_ready = true;
 }
 
-template <typename T>
-const T* EpsDivDivOp::boundary_table(const T* kk, cudaStream_t st)
+namespace {
+size_t boundary_table_values(const DeviceLevel& L) { return static_cast<size_t>(8) * 2 * 10 * L.nl() * L.nl(); }
+}  // namespace
+
+void EpsDivDivOp::alloc_coefficient(DevBuf& buf, int element_size) const
 {
-    DevBuf& buf = std::is_same<T, double>::value ? bdiag64 : bdiag32;
-    if (buf.get() == nullptr) {
+    const size_t n = static_cast<size_t>(q0 ? lvl().cells() : lvl().nodes());
+    buf.alloc(n * element_size, boundary_table_values(lvl()) * element_size);
+}
+
+template <typename T>
+const T* EpsDivDivOp::boundary_table(cudaStream_t st)
+{
+    const bool    own   = (precision == 0) == std::is_same<T, double>::value;
+    const DevBuf& buf   = own ? k : k32;
+    bool&         ready = own ? bdiag_ready : bdiag32_ready;
+    T*            table = static_cast<T*>(buf.tail());
+    if (!ready) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         cuda_check(cudaStreamIsCapturing(st, &cap), "capture status");
         if (cap != cudaStreamCaptureStatusNone)
             throw Error(kErrState, "the operator's boundary table must be built before stream capture");
         const DeviceLevel& L = lvl();
-        DevBuf             b(sizeof(T) * 8 * 2 * 10 * static_cast<size_t>(L.nl()) * L.nl());
+        if (buf.tail_size() < boundary_table_values(L) * sizeof(T))
+            throw Error(kErrState, "a coefficient without room for its boundary table");
+        const T* kk = buf.as<T>();
         if (edd_boundary_table<T>(L.nl(), L.nr(), L.coords<double>(), L.colgeo<double>(), L.radgeo<double>(),
-                                  q0 ? nullptr : kk, q0 ? kk : nullptr, b.as<T>(), st) != 0)
+                                  q0 ? nullptr : kk, q0 ? kk : nullptr, table, st) != 0)
             throw Error(kErrCuda, "boundary table launch failed");
         cuda_check(cudaStreamSynchronize(st), "boundary table");
-        buf = std::move(b);
+        ready = true;
     }
-    return buf.as<T>();
+    return table;
 }
 
 void EpsDivDivOp::prepare_boundary(cudaStream_t st)
 {
     if (precision == 0)
-        (void)boundary_table<double>(k.as<double>(), st);
+        (void)boundary_table<double>(st);
     else
-        (void)boundary_table<float>(k.as<float>(), st);
+        (void)boundary_table<float>(st);
 }
 
 void EpsDivDivOp::prepare_apply(bool need32, cudaStream_t st)
@@ -512,7 +528,7 @@ void EpsDivDivOp::apply_t(const T* const* src, T* const* dst, cudaStream_t st, b
     p.lateral = L.lateral<T>();
     p.colgeo  = L.colgeo<T>();
     p.radgeo  = L.radgeo<T>();
-    if (!diagonal) p.boundary = boundary_table<T>(kk, st);
+    if (!diagonal) p.boundary = boundary_table<T>(st);
     if (q0)
         p.kq0 = kk;
     else

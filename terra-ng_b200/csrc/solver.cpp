@@ -165,7 +165,7 @@ VelocityMultigrid::VelocityMultigrid(const Shell* sh, const EpsDivDivOp& fine, c
     // finest: copy of the caller's operator
     {
         auto op = make_op(fine_);
-        op->k.alloc(fine.k.size());
+        op->alloc_coefficient(op->k, sizeof(double));
         cuda_check(cudaMemcpyAsync(op->k.get(), fine.k.get(), fine.k.size(), cudaMemcpyDeviceToDevice, st),
                    "copy coefficient");
         op->tile_y  = fine.tile_y;
@@ -194,11 +194,10 @@ VelocityMultigrid::VelocityMultigrid(const Shell* sh, const EpsDivDivOp& fine, c
         } else {
             const DeviceLevel& Lc = sh->level(l);
             const auto&        kf = ops64_[l + 1]->k;
+            op->alloc_coefficient(op->k, sizeof(double));
             if (op->q0) {
-                op->k.alloc(sizeof(double) * Lc.cells());
                 chk(cell_coefficient_average(Lc.nl(), Lc.nr(), kf.as<double>(), op->k.as<double>(), st), "coarsen");
             } else {
-                op->k.alloc(sizeof(double) * Lc.nodes());
                 chk(coefficient_inject(Lc.nl(), Lc.nr(), kf.as<double>(), op->k.as<double>(), false, st), "inject");
             }
             if (o.gca == 2) {
@@ -240,7 +239,7 @@ VelocityMultigrid::VelocityMultigrid(const Shell* sh, const EpsDivDivOp& fine, c
             op->tile_y    = ops64_[l]->tile_y;
             op->chunk_x   = ops64_[l]->chunk_x;
             const int64_t n = static_cast<int64_t>(ops64_[l]->k.size() / sizeof(double));
-            op->k.alloc(sizeof(float) * n);
+            op->alloc_coefficient(op->k, sizeof(float));
             chk(convert_f64_to_f32(n, ops64_[l]->k.as<double>(), op->k.as<float>(), st), "convert coefficient");
             ops32_[l] = std::move(op);
         }
@@ -721,7 +720,7 @@ StokesSolver::StokesSolver(const Shell* sh, int vlevel, const double* eta_nodal,
     setup(BT_);
     K_.A.q0              = eta_cell != nullptr;
     const size_t kbytes  = sizeof(double) * (K_.A.q0 ? Lu.cells() : Lu.nodes());
-    K_.A.k.alloc(kbytes);
+    K_.A.alloc_coefficient(K_.A.k, sizeof(double));
     cuda_check(cudaMemcpyAsync(K_.A.k.get(), K_.A.q0 ? static_cast<const void*>(eta_cell) : eta_nodal, kbytes,
                                cudaMemcpyDeviceToDevice, st),
                "copy viscosity");
@@ -1157,7 +1156,7 @@ VelocitySolver::VelocitySolver(const Shell* sh, int level, const double* eta_nod
     A_.bc_surf           = bc_surf;
     A_.q0                = eta_cell != nullptr;
     const size_t kbytes  = sizeof(double) * (A_.q0 ? L.cells() : L.nodes());
-    A_.k.alloc(kbytes);
+    A_.alloc_coefficient(A_.k, sizeof(double));
     cuda_check(cudaMemcpyAsync(A_.k.get(), A_.q0 ? static_cast<const void*>(eta_cell) : eta_nodal, kbytes,
                                cudaMemcpyDeviceToDevice, st),
                "copy viscosity");

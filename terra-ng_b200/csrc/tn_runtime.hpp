@@ -46,34 +46,37 @@ class DevBuf {
     ~DevBuf() { release(); }
     DevBuf(const DevBuf&)            = delete;
     DevBuf& operator=(const DevBuf&) = delete;
-    DevBuf(DevBuf&& o) noexcept : p_(o.p_), n_(o.n_)
+    DevBuf(DevBuf&& o) noexcept : p_(o.p_), n_(o.n_), tail_(o.tail_)
     {
         o.p_ = nullptr;
-        o.n_ = 0;
+        o.n_ = o.tail_ = 0;
     }
     DevBuf& operator=(DevBuf&& o) noexcept
     {
         if (this != &o) {
             release();
-            p_   = o.p_;
-            n_   = o.n_;
-            o.p_ = nullptr;
-            o.n_ = 0;
+            p_    = o.p_;
+            n_    = o.n_;
+            tail_ = o.tail_;
+            o.p_  = nullptr;
+            o.n_ = o.tail_ = 0;
         }
         return *this;
     }
-    void alloc(size_t bytes)
+    // tail: room for a second array behind the first, in the same allocation
+    void alloc(size_t bytes, size_t tail = 0)
     {
         release();
         if (bytes == 0) return;
         // pad to 256 bytes so 16-byte-rounded bulk reads never leave the allocation
-        const size_t padded = (bytes + 255) / 256 * 256;
-        if (cudaMalloc(&p_, padded) != cudaSuccess) {
+        const size_t total = padded(bytes) + padded(tail);
+        if (cudaMalloc(&p_, total) != cudaSuccess) {
             cudaGetLastError();
             p_ = nullptr;
-            throw Error(kErrAlloc, "cudaMalloc of " + std::to_string(padded) + " bytes failed");
+            throw Error(kErrAlloc, "cudaMalloc of " + std::to_string(total) + " bytes failed");
         }
-        n_ = bytes;
+        n_    = bytes;
+        tail_ = tail;
     }
     // alloc unless the buffer already has exactly this size (a rebuild reuses it)
     void ensure(size_t bytes)
@@ -84,7 +87,7 @@ class DevBuf {
     {
         if (p_) cudaFree(p_);
         p_ = nullptr;
-        n_ = 0;
+        n_ = tail_ = 0;
     }
     template <typename T>
     T* as() const
@@ -93,10 +96,14 @@ class DevBuf {
     }
     void*  get() const { return p_; }
     size_t size() const { return n_; }
+    void*  tail() const { return tail_ ? static_cast<char*>(p_) + padded(n_) : nullptr; }
+    size_t tail_size() const { return tail_; }
 
   private:
+    static size_t padded(size_t bytes) { return (bytes + 255) / 256 * 256; }
+
     void*  p_ = nullptr;
-    size_t n_ = 0;
+    size_t n_ = 0, tail_ = 0;
 };
 
 template <typename T>
@@ -239,11 +246,14 @@ struct Operator {
 // matrices instead of the coefficient; boundary conditions are baked into a
 // copy of the matrices the first time an apply needs them.
 struct EpsDivDivOp : Operator {
-    DevBuf k;  // nodal or cell coefficient in `precision` (may be empty in stored mode)
+    // nodal or cell coefficient in `precision` (may be empty in stored mode); behind it, and behind k32, the boundary
+    // rows' diagonals of that coefficient (edd_boundary_table): an allocation of their own made every operator 0.1 to
+    // 0.5 ms slower to create
+    DevBuf k;
     bool   q0 = false;
     bool   diagonal = false;
     int    tile_y = 0, chunk_x = 0;
-    DevBuf bdiag64, bdiag32;  // boundary rows' diagonals of k (edd_boundary_table), per apply precision
+    bool   bdiag_ready = false, bdiag32_ready = false;  // the tables behind k and k32 are built
 
     // free slip on both boundaries: the orthonormal rotation modes as coefficients over the raw modes e_i x X
     // (evaluated from the coordinates by the kernels) and the scratch of the penalty dst += eps sum_i (n_i^T src) n_i
@@ -282,9 +292,10 @@ struct EpsDivDivOp : Operator {
     template <typename T>
     void vjp_logeta(const T* const* u, const T* const* lam, T* grad_cell, cudaStream_t st) const;
     // free-slip/free-slip null-space penalty (epsilon_divdiv_kerngen.hpp:324-445, :711-785)
-    // builds the boundary table of an apply in T with coefficient kk (synchronous; no-op once built)
+    // builds the boundary table of an apply in T (synchronous; no-op once built)
     template <typename T>
-    const T* boundary_table(const T* kk, cudaStream_t st);
+    const T* boundary_table(cudaStream_t st);
+    void alloc_coefficient(DevBuf& buf, int element_size) const;  // k or k32, with room for its table
     void prepare_boundary(cudaStream_t st);  // the table of the operator's own precision
     // everything a (non-diagonal) apply builds on first use, so that it can be captured (synchronous); need32: FP32
     // applies of the stored matrices too
