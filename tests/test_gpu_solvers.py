@@ -592,12 +592,12 @@ def test_gram_schmidt_against_vector_by_vector(cuda, lat, rad, restart):
     assert np.abs(np.array(hist) - np.array(ref)).max() < 1e-8
 
 
-@pytest.mark.parametrize("lat,rad", [(1, 1), (2, 1), (1, 4), (2, 2), (3, 3)])
+@pytest.mark.parametrize("lat,rad", [(1, 1), (2, 1), (1, 4), (2, 2), (3, 3), (4, 4)])
 @pytest.mark.parametrize("bcs", [(1, 2), (0, 1), (2, 2)])
 def test_compact_store_radial_layers(cuda, lat, rad, bcs):
-    """Stored matrices without their null space: levels of two layers (edge cells only), three and more, and one wider
-    than a block. The stored element matrices give the matrix-free operator, in FP64 and, for the same matrices behind an
-    FP32 operator, in FP32; bounds as in the tests above. Rebuilding after a change of boundary conditions too."""
+    """Stored matrices without their null space, in FP64: levels of two layers (edge cells only), four and more, one wider
+    than a block, and one whose store of 83 MB is read with evict-first. The stored element matrices give the matrix-free
+    operator; bounds as in the tests above. Rebuilding after a change of boundary conditions too."""
     import torch
 
     sh = O.Shell(lat, rad)
@@ -612,6 +612,28 @@ def test_compact_store_radial_layers(cuda, lat, rad, bcs):
         op.apply(_t(u), out)
         ref = O.EpsDivDiv(sh, k=k, bc_cmb=b[0], bc_surface=b[1]).apply(u, path="slow")
         assert rel_err(out.cpu().numpy(), ref) < 1e-12
+
+
+@pytest.mark.parametrize("lat,rad,nlev", [(2, 3, 3), (2, 5, 3), (4, 3, 3), (6, 5, 5)])
+@pytest.mark.parametrize("bcs", [(1, 1), (1, 2)])
+def test_compact_store_fp32(cuda, lat, rad, nlev, bcs):
+    """The FP32 copies of the compact store, which only the FP32 V-cycle reads: Galerkin levels of two blocks, of several
+    and, at (5, 4), a store of 166 MB read with evict-first. The FP32 cycle against the FP64 one of the same
+    hierarchy; FP32 rounds to 6e-8, and 4e-6 is some 60 roundings in one direction (a cycle makes about 60 updates)."""
+    import torch
+
+    g = T.Shell(lat, rad, num_levels=nlev)
+    nl, nr = g.dims(-1)
+    k = torch.tensor(O.Shell(lat, rad).coords[..., 0], device=cuda).exp()[..., None].expand(10, nl, nl, nr).contiguous()
+    s = T.VelocitySolver(g, eta=k, bc_cmb=bcs[0], bc_surface=bcs[1], mixed_precision=1, coarse_solver=T.COARSE_DENSE)
+    b = T.stokes_rhs_enforce(g, -1, T.random_vector(g, nlev - 1, 3, 8), *bcs)
+    out = []
+    for dt in (torch.float64, torch.float32):
+        x = torch.zeros(b.shape, dtype=dt, device=cuda)
+        s.vcycle(x, b.to(dt))
+        out.append(x.double())
+    assert torch.isfinite(out[1]).all()
+    assert ((out[1] - out[0]).norm() / out[0].norm()).item() < 4e-6
 
 
 @pytest.mark.parametrize("lat,rad", [(1, 2), (2, 2), (2, 3), (3, 2)])
@@ -635,10 +657,10 @@ def test_fast_gca_build_equals_plain_build(cuda, lat, rad, q0, interpolation):
     assert rel_err(mats[0], mats[1]) < 1e-13
 
 
-@pytest.mark.parametrize("lat,rad,nlev", [(1, 2, 2), (1, 3, 2), (2, 2, 2), (3, 2, 2), (3, 3, 2), (3, 3, 3), (3, 4, 2), (4, 4, 2)])
+@pytest.mark.parametrize("lat,rad,nlev", [(1, 2, 2), (1, 3, 2), (2, 2, 2), (3, 2, 2), (3, 3, 2), (3, 3, 3), (3, 4, 2)])
 def test_coarse_cg_equals_dense_solve(cuda, lat, rad, nlev):
     """The coarsest CG run to convergence against the dense solve, on coarsest levels of a few nodes a CTA (and CTAs
-    without any), with rows in shared memory, and too large for the row kernel: the V-cycles agree to the CG's 1e-13
+    without any), with rows in shared memory, and, at (2, 3), with rows read from L2: the V-cycles agree to the CG's 1e-13
     times the conditioning of the level (1e-9, as against the oracle)."""
     import torch
 
@@ -649,14 +671,28 @@ def test_coarse_cg_equals_dense_solve(cuda, lat, rad, nlev):
     b = O.enforce_rhs_bcs(sh, consistent(sh, O.seeded_normal(sh.vec_shape, 30)), 1, 2)
     res = []
     for kw in ({"coarse_solver": T.COARSE_DENSE}, {"coarse_relative_tolerance": 1e-13, "coarse_max_iterations": 4000}):
-        try:
-            s = T.VelocitySolver(g, eta=_t(k), bc_cmb=1, bc_surface=2, **kw)
-        except T.TerraError:  # the dense solve has a size limit
-            pytest.skip("coarsest level too large for the dense solve")
+        s = T.VelocitySolver(g, eta=_t(k), bc_cmb=1, bc_surface=2, **kw)
         x = torch.zeros(sh.vec_shape, dtype=torch.float64, device=cuda)
         s.vcycle(x, _t(b))
         res.append(x.cpu().numpy())
     assert rel_err(res[1], res[0]) < 1e-9
+
+
+def test_coarse_cg_over_element_matrices(cuda):
+    """A coarsest level too large for the row kernel (the six vector components of 5778 nodes take 277 KB of the 200 KB
+    of shared memory a block may use) and for the dense solve: CG over the stored element matrices, run to convergence,
+    against the oracle's cycle (1e-9, as in the cycles above)."""
+    import torch
+
+    level, bcs = 4, (1, 2)
+    sh, k, g, solver, H = _hierarchy(level, 2, bcs, 1, coarse_relative_tolerance=1e-13, coarse_max_iterations=4000)
+    b = O.enforce_rhs_bcs(sh, consistent(sh, O.seeded_normal(sh.vec_shape, 34)), *bcs)
+    ref = H.multigrid().solve(np.zeros(sh.vec_shape), b)
+    x = torch.zeros(sh.vec_shape, dtype=torch.float64, device=cuda)
+    solver.vcycle(x, _t(b))
+    assert rel_err(x.cpu().numpy(), ref) < 1e-9
+    its, init, final = solver.coarse_stats()
+    assert 0 < its < 4000 and final <= 1e-13 * init
 
 
 @pytest.mark.parametrize("gca", [0, 1, 2])
