@@ -3,9 +3,9 @@
 //   d(lambda^T A u) / d log(eta_cell) = lambda_e^T A_e(eta_cell) u_e,
 // the cell's own contribution to the bilinear form with the operator's
 // boundary treatment (Dirichlet masks, free-slip projection and normal
-// stiffness). One thread per cell; the cell math is the one the matrix-free
-// kernel uses (tn_wedge_math.cuh), accumulated and reduced in the working
-// precision T. The velocity part of the backward pass, A^T lambda = A lambda,
+// stiffness). One thread per cell; the cell's forces (tn_wedge_math.cuh; the
+// matrix-free apply has arithmetic of its own) are accumulated and reduced in
+// the working precision T. The velocity part of the backward pass, A^T lambda = A lambda,
 // is the forward apply itself (A is symmetric).
 #include "tn_device.cuh"
 #include "tn_kernels.hpp"
@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(128) vjp_logeta_kernel(VjpLaunch<T> A)
     const T alpha = T(0.5) / rm, beta = T(1) / (T(6) * hdr);
     const T dfac  = rm * rm * hdr;  // Q0: the cell value multiplies the wedge volume directly
 
-    T   u[4][2][3], lam[4][2][3], out[4][2][3], nrm[4][3], ks[4];
+    T   u[4][2][3], lam[4][2][3], out[4][2][3], nrm[4][3];
     int bcs[2] = {r == 0 ? A.bc_cmb : 0, r + 1 == nr - 1 ? A.bc_surf : 0};
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -44,7 +44,6 @@ __global__ void __launch_bounds__(128) vjp_logeta_kernel(VjpLaunch<T> A)
         const T   m  = sqrt(c[0] * c[0] + c[1] * c[1] + c[2] * c[2]);
 #pragma unroll
         for (int k = 0; k < 3; ++k) nrm[q][k] = c[k] / m;
-        ks[q] = T(0);
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
             const int64_t id = node_index(nl, nr, d, qx, qy, r + s);
@@ -57,7 +56,7 @@ __global__ void __launch_bounds__(128) vjp_logeta_kernel(VjpLaunch<T> A)
         }
     }
     const T kcell = A.kq0[cell];
-    cell_apply<T, false>(u, ks, kcell, true, geo, alpha, beta, dfac, bcs, nrm, out);
+    cell_apply<T>(u, kcell, geo, alpha, beta, dfac, bcs, nrm, out);
     T acc = T(0);
 #pragma unroll
     for (int q = 0; q < 4; ++q)

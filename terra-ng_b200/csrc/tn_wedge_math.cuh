@@ -1,5 +1,4 @@
-// Per-cell wedge math of the epsilon-div-div operator, shared by the CUDA
-// kernels and host-side unit checks (__host__ __device__).
+// Per-cell wedge math of the epsilon-div-div operator (kernel_helpers.hpp:179-312), shared by the CUDA kernels.
 #pragma once
 
 #include <cmath>
@@ -90,14 +89,11 @@ __host__ __device__ void trafo_nt(const T n[3], T R[3][3])
     }
 }
 
-// One hex cell (two wedges). u[q][s][c]: corner q, side s (0 bottom, 1 top).
-// ks[q]: k_bot + k_top (nodal) ; kcell used when Q0. Accumulates into out.
-// bcs[s]: boundary condition of side s of this cell (0: interior/Neumann,
-// 1: Dirichlet, 2: free-slip).
-template <typename T, bool DIAG>
-__host__ __device__ __forceinline__ void cell_apply(const T (&u)[4][2][3], const T (&ks)[4], T kcell, bool q0, const T* geo,
-                                           T alpha, T beta, T dfac, const int (&bcs)[2], const T (&nrm)[4][3],
-                                           T (&out)[4][2][3])
+// One hex cell (two wedges) with a coefficient of its own. u[q][s][c]: corner q, side s (0 bottom, 1 top). Accumulates
+// into out. bcs[s]: boundary condition of side s of this cell (0: interior/Neumann, 1: Dirichlet, 2: free-slip).
+template <typename T>
+__host__ __device__ __forceinline__ void cell_apply(const T (&u)[4][2][3], T kcell, const T* geo, T alpha, T beta, T dfac,
+                                                    const int (&bcs)[2], const T (&nrm)[4][3], T (&out)[4][2][3])
 {
     const bool fs_any = (bcs[0] == 2) || (bcs[1] == 2);
     T          uin[4][2][3];
@@ -129,8 +125,7 @@ __host__ __device__ __forceinline__ void cell_apply(const T (&u)[4][2][3], const
     for (int w = 0; w < 2; ++w) {
         const T* gw = geo + 10 * w;
         const int q0i = wedge_corner(w, 0), q1i = wedge_corner(w, 1), q2i = wedge_corner(w, 2);
-        const T   kv  = q0 ? kcell : (ks[q0i] + ks[q1i] + ks[q2i]);
-        const T   kw  = kv * gw[9] * dfac;
+        const T   kw  = kcell * gw[9] * dfac;
         T         E1[3], E2[3], E3[3];
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
@@ -138,64 +133,60 @@ __host__ __device__ __forceinline__ void cell_apply(const T (&u)[4][2][3], const
             E2[i] = alpha * gw[3 + i];
             E3[i] = beta * gw[6 + i];
         }
-        if (!DIAG) {
-            T a[3], b[3], D[3];
+        T a[3], b[3], D[3];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const T S0 = uin[q0i][0][c] + uin[q0i][1][c];
-                const T S1 = uin[q1i][0][c] + uin[q1i][1][c];
-                const T S2 = uin[q2i][0][c] + uin[q2i][1][c];
-                a[c]       = S1 - S0;
-                b[c]       = S2 - S0;
-                D[c]       = (uin[q0i][1][c] - uin[q0i][0][c]) + (uin[q1i][1][c] - uin[q1i][0][c]) +
-                       (uin[q2i][1][c] - uin[q2i][0][c]);
+        for (int c = 0; c < 3; ++c) {
+            const T S0 = uin[q0i][0][c] + uin[q0i][1][c];
+            const T S1 = uin[q1i][0][c] + uin[q1i][1][c];
+            const T S2 = uin[q2i][0][c] + uin[q2i][1][c];
+            a[c]       = S1 - S0;
+            b[c]       = S2 - S0;
+            D[c]       = (uin[q0i][1][c] - uin[q0i][0][c]) + (uin[q1i][1][c] - uin[q1i][0][c]) +
+                   (uin[q2i][1][c] - uin[q2i][0][c]);
+        }
+        // G[i][j] = d_i u_j
+        T G[3][3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) G[i][j] = E1[i] * a[j] + E2[i] * b[j] + E3[i] * D[j];
+        const T div = G[0][0] + G[1][1] + G[2][2];
+        const T k2  = T(2) * kw;
+        const T kd  = kw * (T(2) / T(3)) * div;
+        const T s00 = k2 * G[0][0] - kd, s11 = k2 * G[1][1] - kd, s22 = k2 * G[2][2] - kd;
+        const T s01 = kw * (G[0][1] + G[1][0]), s02 = kw * (G[0][2] + G[2][0]), s12 = kw * (G[1][2] + G[2][1]);
+        T       v1[3], v2[3], wv[3];
+        v1[0] = s00 * E1[0] + s01 * E1[1] + s02 * E1[2];
+        v1[1] = s01 * E1[0] + s11 * E1[1] + s12 * E1[2];
+        v1[2] = s02 * E1[0] + s12 * E1[1] + s22 * E1[2];
+        v2[0] = s00 * E2[0] + s01 * E2[1] + s02 * E2[2];
+        v2[1] = s01 * E2[0] + s11 * E2[1] + s12 * E2[2];
+        v2[2] = s02 * E2[0] + s12 * E2[1] + s22 * E2[2];
+        wv[0] = s00 * E3[0] + s01 * E3[1] + s02 * E3[2];
+        wv[1] = s01 * E3[0] + s11 * E3[1] + s12 * E3[2];
+        wv[2] = s02 * E3[0] + s12 * E3[1] + s22 * E3[2];
+        const bool bot_on = bcs[0] != 1, top_on = bcs[1] != 1;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const T v0 = -(v1[c] + v2[c]);
+            if (bot_on) {
+                out[q0i][0][c] += v0 - wv[c];
+                out[q1i][0][c] += v1[c] - wv[c];
+                out[q2i][0][c] += v2[c] - wv[c];
             }
-            // G[i][j] = d_i u_j
-            T G[3][3];
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-#pragma unroll
-                for (int j = 0; j < 3; ++j) G[i][j] = E1[i] * a[j] + E2[i] * b[j] + E3[i] * D[j];
-            const T div = G[0][0] + G[1][1] + G[2][2];
-            const T k2  = T(2) * kw;
-            const T kd  = kw * (T(2) / T(3)) * div;
-            const T s00 = k2 * G[0][0] - kd, s11 = k2 * G[1][1] - kd, s22 = k2 * G[2][2] - kd;
-            const T s01 = kw * (G[0][1] + G[1][0]), s02 = kw * (G[0][2] + G[2][0]), s12 = kw * (G[1][2] + G[2][1]);
-            T       v1[3], v2[3], wv[3];
-            v1[0] = s00 * E1[0] + s01 * E1[1] + s02 * E1[2];
-            v1[1] = s01 * E1[0] + s11 * E1[1] + s12 * E1[2];
-            v1[2] = s02 * E1[0] + s12 * E1[1] + s22 * E1[2];
-            v2[0] = s00 * E2[0] + s01 * E2[1] + s02 * E2[2];
-            v2[1] = s01 * E2[0] + s11 * E2[1] + s12 * E2[2];
-            v2[2] = s02 * E2[0] + s12 * E2[1] + s22 * E2[2];
-            wv[0] = s00 * E3[0] + s01 * E3[1] + s02 * E3[2];
-            wv[1] = s01 * E3[0] + s11 * E3[1] + s12 * E3[2];
-            wv[2] = s02 * E3[0] + s12 * E3[1] + s22 * E3[2];
-            const bool bot_on = bcs[0] != 1, top_on = bcs[1] != 1;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const T v0 = -(v1[c] + v2[c]);
-                if (bot_on) {
-                    out[q0i][0][c] += v0 - wv[c];
-                    out[q1i][0][c] += v1[c] - wv[c];
-                    out[q2i][0][c] += v2[c] - wv[c];
-                }
-                if (top_on) {
-                    out[q0i][1][c] += v0 + wv[c];
-                    out[q1i][1][c] += v1[c] + wv[c];
-                    out[q2i][1][c] += v2[c] + wv[c];
-                }
+            if (top_on) {
+                out[q0i][1][c] += v0 + wv[c];
+                out[q1i][1][c] += v1[c] + wv[c];
+                out[q2i][1][c] += v2[c] + wv[c];
             }
         }
-        // Diagonal terms: all nodes in DIAG mode, Dirichlet-side nodes otherwise;
-        // free-slip normal stiffness Ann on free-slip sides.
-        const bool need_diag = DIAG || bcs[0] == 1 || bcs[1] == 1;
-        if (need_diag || fs_any) {
+        // Diagonal terms of Dirichlet sides, normal stiffness Ann of free-slip sides.
+        if (bcs[0] == 1 || bcs[1] == 1 || fs_any) {
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
                 const bool dir_side = bcs[s] == 1;
                 const bool fs_side  = bcs[s] == 2;
-                if (!(DIAG || dir_side || fs_side)) continue;
+                if (!(dir_side || fs_side)) continue;
                 const T sg = s == 0 ? T(-1) : T(1);
 #pragma unroll
                 for (int m = 0; m < 3; ++m) {
@@ -209,21 +200,7 @@ __host__ __device__ __forceinline__ void cell_apply(const T (&u)[4][2][3], const
                     const T gg = g[0] * g[0] + g[1] * g[1] + g[2] * g[2];
                     if (fs_side) {
                         const T ng = nrm[q][0] * g[0] + nrm[q][1] * g[1] + nrm[q][2] * g[2];
-                        if (!DIAG) {
-                            ann[q][s] += kw * (gg + ng * ng * (T(1) / T(3)));
-                        } else {
-                            T R[3][3];
-                            trafo_nt(nrm[q], R);
-                            T v[3];
-#pragma unroll
-                            for (int a_ = 0; a_ < 3; ++a_) {
-                                const T Rg = R[a_][0] * g[0] + R[a_][1] * g[1] + R[a_][2] * g[2];
-                                const T Rs = R[a_][0] * u[q][s][0] + R[a_][1] * u[q][s][1] + R[a_][2] * u[q][s][2];
-                                v[a_]      = kw * (gg + Rg * Rg * (T(1) / T(3))) * Rs;
-                            }
-#pragma unroll
-                            for (int c = 0; c < 3; ++c) out[q][s][c] += R[0][c] * v[0] + R[1][c] * v[1] + R[2][c] * v[2];
-                        }
+                        ann[q][s] += kw * (gg + ng * ng * (T(1) / T(3)));
                     } else {
 #pragma unroll
                         for (int c = 0; c < 3; ++c)
@@ -234,7 +211,7 @@ __host__ __device__ __forceinline__ void cell_apply(const T (&u)[4][2][3], const
         }
     }
 
-    if (!DIAG && fs_any) {
+    if (fs_any) {
         // test-side projection and normal stiffness: o <- P o + Ann (n.u) n
 #pragma unroll
         for (int s = 0; s < 2; ++s) {
