@@ -218,7 +218,8 @@ void EpsDivDivOp::finish_selective(cudaStream_t st)
     const DeviceLevel& L = lvl();
     if (!selective) throw Error(kErrState, "the operator has no selective storage");
     sel_delta.ensure(static_cast<size_t>(mats_values()) * sizeof(double));
-    if (element_matrices(L.nl(), L.nr(), L.coords<double>(), L.radii<double>(), q0 ? nullptr : k.as<double>(),
+    if (sel_count > 0 &&
+        element_matrices(L.nl(), L.nr(), L.coords<double>(), L.radii<double>(), q0 ? nullptr : k.as<double>(),
                          q0 ? k.as<double>() : nullptr, sel_delta.as<double>(), st, sel_cells.as<int>(), sel_count,
                          mats.as<double>()) != 0)
         throw Error(kErrCuda, "correction matrix launch failed");
@@ -337,6 +338,11 @@ void gca_coarsen(const EpsDivDivOp& fine, EpsDivDivOp& coarse, cudaStream_t st, 
     if (coarse.selective) {
         sl.cells  = coarse.sel_cells.as<int>();
         sl.nslots = coarse.sel_count;
+    }
+    if (coarse.selective && coarse.sel_count == 0) {  // no marked cell: nothing to build (a null slot list means all cells)
+        coarse.mats.release();
+        coarse.finish_selective(st);
+        return;
     }
     sl.err = coarse.shell->err_word();
     coarse.mats.ensure(static_cast<size_t>(coarse.mats_values()) * sizeof(double));

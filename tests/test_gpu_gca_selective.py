@@ -186,3 +186,50 @@ def test_fp32_vcycle_freeslip_both(cuda, case, gca):
     s32.vcycle(x32, _t(b, torch.float32))
     assert rel_err(x32.double().cpu().numpy(), x64.cpu().numpy()) < 1e-4
     assert g.check_device_error() == 0
+
+
+@pytest.mark.parametrize("nlev", [2, 3])
+@pytest.mark.parametrize("mixed", [0, 1])
+def test_no_marked_cell(cuda, nlev, mixed):
+    """A viscosity that marks no cell (a uniform one): no level stores anything and the hierarchy is the rediscretised one
+    of gca = 0. Both run the same kernels on the same numbers up to the coarsest level, whose matrices the two assemble by
+    the same kernel: cycles equal to rounding in FP64 (1e-12) and in FP32 (4e-6, as between precisions elsewhere)."""
+    import torch
+
+    g = T.Shell(3, num_levels=nlev)
+    nl, nr = g.dims(-1)
+    k = torch.full((10, nl, nl, nr), 2.5, dtype=torch.float64, device=cuda)
+    b = T.stokes_rhs_enforce(g, -1, T.random_vector(g, nlev - 1, 3, 9), 1, 2)
+    out = []
+    for gca in (2, 0):
+        s = T.VelocitySolver(g, eta=k, bc_cmb=1, bc_surface=2, gca=gca, mixed_precision=mixed,
+                             coarse_solver=T.COARSE_DENSE)
+        if gca == 2:
+            assert [s.level_storage(l)[0] for l in range(1, nlev)] == [0] * (nlev - 1)
+        x = torch.zeros_like(b, dtype=torch.float32 if mixed else torch.float64)
+        s.vcycle(x, b.to(x.dtype))
+        out.append(x.double())
+    assert torch.isfinite(out[0]).all()
+    assert ((out[0] - out[1]).norm() / out[1].norm()).item() < (4e-6 if mixed else 1e-12)
+
+
+def test_no_marked_cell_operator(cuda):
+    """The same through the operator-level API: a selective operator without cells applies as the matrix-free one."""
+    import torch
+
+    g = T.Shell(3, num_levels=2)
+    k = [_t(smooth_viscosity(O.Shell(l), 4, 10.0)) for l in (3, 2)]
+    fine = T.EpsDivDiv(g, 1, k=k[0], bc_cmb=1, bc_surface=2)
+    coarse = T.EpsDivDiv(g, 0, k=k[1], bc_cmb=1, bc_surface=2)
+    nl, nr = g.dims(0)
+    u = T.random_vector(g, 0, 3, 10)
+    ref, out = torch.zeros_like(u), torch.zeros_like(u)
+    coarse.apply(u, ref)
+    coarse.set_selective_matrices(0, torch.zeros((10, nl - 1, nl - 1, nr - 1), dtype=torch.uint8, device=cuda))
+    T.gca_build(fine, coarse)
+    assert coarse.stored_cells()[0] == 0
+    coarse.apply(u, out)
+    assert torch.equal(out, ref)
+    coarse.set_diagonal(True)
+    coarse.apply(u, out)
+    assert torch.isfinite(out).all()
