@@ -32,12 +32,15 @@ struct PtrSet {
 // load hangs on another (masks and values are read together, the mask applied after), and components run in
 // different threads. Before (components in a loop of run-time length, loads behind the ownership test), cold caches:
 // restriction 42 / 19 / 18 us to level 5 / 4 / 3 in FP32, prolongation 38 us to level 6. With the residual formed in the
-// restriction instead of a pass of its own the level-6 mixed preconditioner went from 3.55 to 3.52 ms.
+// restriction instead of a pass of its own the level-6 mixed preconditioner went from 3.55 to 3.52 ms. The pointer set is a
+// __grid_constant__: indexed by blockIdx.y, a plain parameter is copied to the stack by every thread (prolongation of three
+// components to level 6: FP32 102 us instead of 34, FP64 107 instead of 37; a loop over the components in the thread 37 / 47).
 constexpr int kTransferThreads = 256;
 
 template <typename T>
-__global__ void __launch_bounds__(kTransferThreads) prolongate_kernel(int nlf, int nrf, PtrSet<T> P, int n, Decoder rad,
-                                                                      Decoder lat)
+__global__ void __launch_bounds__(kTransferThreads) prolongate_kernel(int nlf, int nrf,
+                                                                      const __grid_constant__ PtrSet<T> P, int n,
+                                                                      Decoder rad, Decoder lat)
 {
     const int nlc = (nlf + 1) / 2, nrc = (nrf + 1) / 2;
     const int i   = blockIdx.x * blockDim.x + threadIdx.x;
@@ -70,7 +73,8 @@ __global__ void __launch_bounds__(kTransferThreads) prolongate_kernel(int nlf, i
 // RESIDUAL: restricts b - in instead of in.
 template <typename T, bool RESIDUAL>
 __global__ void __launch_bounds__(kTransferThreads) restrict_kernel(int nlf, int nrf, const uint8_t* __restrict__ owned,
-                                                                    PtrSet<T> P, int n, Decoder rad, Decoder lat)
+                                                                    const __grid_constant__ PtrSet<T> P, int n,
+                                                                    Decoder rad, Decoder lat)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     chain_enter();
