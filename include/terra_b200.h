@@ -131,7 +131,9 @@ int tn_operator_set_diagonal(tn_operator* op, int diagonal);
  * 324-445, :711-785); the modes are built by the first apply or this call
  * (synchronous, before any stream capture). */
 int tn_operator_set_boundary_conditions(tn_operator* op, int bc_cmb, int bc_surface);
-/* Override the CTA tile (0 = default); for tuning. */
+/* Launch shape of the matrix-free apply, for tuning (0 = default). tile_y (0..7 in FP64, 0..11 in FP32): node lines a
+ * CTA owns, at most what the level's radial layers leave room for (a smaller tile is taken silently). chunk_x (0..64):
+ * rows a CTA takes from the flattened sweep over (diamond, tile, x). */
 int tn_operator_set_tile(tn_operator* op, int tile_y, int chunk_x);
 /* apply_impl: dst = A src (Replace) or dst += A src (Add); with
  * CommunicateAdditively the interface duplicates of dst are summed afterwards.

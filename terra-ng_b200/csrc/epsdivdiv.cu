@@ -42,11 +42,12 @@
 // Every node value is written once by its owner: no atomics, no zeroing pass.
 // Diamond-edge duplicates hold this diamond's partial sums afterwards; the interface-sum kernel completes them.
 //
-// What bounds it: issue, at 420 (FP32) and 480 (FP64) warp instructions per row, half of them floating point. With
+// What bounds it: in FP32 issue (0.70 of the slots), in FP64 the wait for the row barrier and for results with 12 warps
+// (issue 0.49, FP64 pipe 0.46), both at 510 and 570 thread instructions per cell, half of them floating point. With
 // radial sums per cell corner, radial factors and boundary code in every lane and a chunked grid the same apply took
 // 820 / 1070 instructions per cell. Measured on the level-6 apply with interface sum (L2 flushed): FP32 115 -> 69 us,
-// FP64 199 -> 102 us; level 7, FP64, per-cell coefficient: 1291 -> 703 us. Tried and slower: FP32 pairs on the
-// packed FP32x2 instructions (12 warps of 152 registers: half the instructions per cell, but 0.48 instead of 0.70
+// FP64 199 -> 100 us; level 7, FP64, per-cell coefficient: 1.29 -> 0.71 ms. Tried and slower, same measure: FP32 pairs on
+// the packed FP32x2 instructions (12 warps of 152 registers: half the instructions per cell, but 0.48 instead of 0.70
 // issue; 71 us), mbarriers between neighbouring warps instead of the row barrier (79 us FP32, 126 us FP64),
 // 14 FP64 warps of 128 registers (116 us), 20 FP32 warps of 80 registers (71 us).
 #include "tn_device.cuh"
@@ -588,8 +589,8 @@ __global__ void __launch_bounds__(Shape<T>::kThreads, 1) epsdivdiv_kernel(const 
             for (int c = 0; c < 3; ++c) cL[q][c] = cR[q][c] = T(0);
         if (some && x < nl - 1) load_column(slot, o);
         const int cols = min(xe, nl - 1);
-        // FP64 has registers for two columns a trip, which saves copying the column behind (105 -> 102 us at level 6);
-        // FP32 spills with it (69 -> 73 us)
+        // FP64 has registers for two columns a trip, which saves copying the column behind (105 -> 102 us at level 6).
+        // FP32, which spills 36 to 52 bytes at its 72 registers, spills more with it (69 -> 73 us).
 #pragma unroll(sizeof(T) == 8 ? 2 : 1)
         for (; x < cols; ++x, ++f) {
             const uint32_t n1 = slot + 1 == kRing ? 0 : slot + 1;
@@ -834,7 +835,8 @@ EddPlan edd_plan(int nl, int nr, int sms, int tile_y, int chunk_x)
 {
     // Warps come in whole strips. The cost of a shape is rows per CTA (plus the repeated column) times the time of a
     // row: the issue time of its warps, four schedulers at a time, plus a latency floor of about five warps. It picks
-    // 12 strips at level 6 in FP32 (69 us; 11 strips 80 us) and 6 in FP64 (105 us; 4 strips 140 us).
+    // 12 strips at level 6 in FP32 (69 us; 11 strips 80 us) and 6 in FP64 (105 us, with one column a trip; 4 strips
+    // 140 us).
     const int nrc = nr - 1, slots = 32;
     const int wps = nrc > slots ? nrc / slots : 1;  // warps per strip
     const int spw = nrc < slots ? slots / nrc : 1;  // strips per warp

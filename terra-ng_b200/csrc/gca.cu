@@ -420,7 +420,10 @@ __global__ void __launch_bounds__(kMmaThreads) gca_build_mma_kernel(GcaBuildArgs
 // fine wedge each, for all 32 cells, into shared memory (values x lanes, no bank conflicts). Then warp (t, g) sums the
 // entries of two or three node pairs (c, e) of coarse wedge t over the 8 fine wedges it receives, in registers, and
 // writes them: 32 consecutive doubles per value. One CTA of 352 threads per coarse hex, which wrote 342 separate
-// doubles and went through three block barriers for one cell, took 6.4 ms for the 327,680 cells of level 5.
+// doubles and went through three block barriers for one cell, took 6.4 ms for the 327,680 cells of level 5; now 1.72 ms.
+// What bounds it: latency and the load/store queue. 126 registers and 512 threads leave one CTA on an SM, whose two phases
+// overlap with nothing, and the interpolation rows go through 384 bytes of stack. Issue 0.23, FP64 pipe 0.11, DRAM 0.05 of
+// their peaks at 40,960 cells (234 us).
 constexpr int kRankCells  = 32;
 constexpr int kRankWarps  = 16;
 constexpr int kRankGroups = 8;

@@ -346,7 +346,8 @@ __global__ void scale_recip_kernel(int64_t n, T* __restrict__ y, const T* __rest
 // apply, and a pass that wrote A x = 0, the level-6 mixed preconditioner took 3.52 ms instead of 3.16 and the level-4
 // velocity solve 18.8 ms instead of 16.5.
 // STREAM: the vectors that only this kernel touches (b, d, D^-1) pass with evict-first, so that x and A x, which the
-// operator reads and writes around it, stay in L2. Taken where the seven vectors outgrow half of L2: with 16-byte accesses
+// operator reads and writes around it, stay in L2. Taken where a step's five reads and two writes exceed 64 MB, that is
+// from vectors of 9.6 MB on (five of them: 48 MB, with the operator's own data more than L2 keeps): with 16-byte accesses
 // the level-6 mixed preconditioner went from 3.16 to 2.97 ms, and the level-4 velocity solve, whose vectors stay in L2, did
 // not change.
 template <typename T>
@@ -696,8 +697,10 @@ __global__ void __launch_bounds__(kPcgThreads, 1) coarse_pcg_kernel(CoarsePcgArg
 // r sent to all CTAs together with its <r, r>, and p = r + beta p on the full copies: two cluster barriers, both sums in
 // rank order, no atomics.
 //
-// Bound by latency (barriers and reductions). With element matrices, partial vectors summed over distributed shared
-// memory and interface sums, an iteration took 14.5 us at level 2.
+// Bound by latency (block and cluster barriers). Over element matrices, with partial vectors summed over distributed
+// shared memory and interface sums, an iteration takes longer at every size: 14.2 us against 5.5 on level (2, 2) (lateral,
+// radial). Where the rows do not fit they are read from L2 (A.rows_in_smem): level (2, 3) 22.7 -> 9.0 us, (2, 4)
+// 28.7 -> 14.2, (3, 2) 30.1 -> 16.3. Levels whose vectors do not fit either keep the element matrices.
 // ---------------------------------------------------------------------------
 constexpr int kRowLanes = 16;
 
