@@ -580,6 +580,89 @@ __global__ void __launch_bounds__(32 * kRankWarps) gca_build_rank_kernel(GcaBuil
     }
 }
 
+// The same for one coarse hex a CTA, for builds of few cells: the lanes of the kernel above would stay empty, and its chain
+// of one fine wedge a thread is longer than the launch. Here the set-up is spread over the block in two short phases: the
+// 16 x 18 gradients, the 16 weights and the 96 rows of the interpolation matrices; the 16 x 18 entries of h. Thread
+// (t, p) of the first 342 then sums entry p of coarse wedge t over the 8 fine wedges it receives. The lines between the two
+// (one build, nodal coefficient, this kernel / the one above): constant interpolation 80 cells 20 / 39 us, 640 30 / 39,
+// 1280 38 / 40, 2560 60 / 41; linear 80 cells 19 / 55 us, 1280 36 / 56, 2560 55 / 58, 10240 167 / 138.
+constexpr int kHexThreads = 416;
+constexpr int kHexCells   = 1024, kHexCellsLinear = 2560;  // up to here (constant, linear interpolation)
+
+__global__ void __launch_bounds__(kHexThreads, 3) gca_build_hex_kernel(GcaBuildArgs A)
+{
+    const int nlf = A.nlf, nrf = A.nrf;
+    int       slot, d, xc, yc, rc;
+    if (!coarse_cell_of_block(A, slot, d, xc, yc, rc)) return;
+
+    __shared__ double P[kFineWedges][6][6];
+    __shared__ double G[kFineWedges][6][3];
+    __shared__ double H[kFineWedges][6][3];
+    __shared__ double kw[kFineWedges];
+
+    const int  tid    = threadIdx.x;
+    const auto column = [&](int h) {  // geometry of the fine column of hex h
+        return A.colgeo + ((static_cast<int64_t>(d) * (nlf - 1) + 2 * xc + (h & 1)) * (nlf - 1) + 2 * yc + (h >> 1 & 1)) * 20;
+    };
+    if (tid < kFineWedges * 18) {
+        // gradient component c of shape function n of fine wedge f
+        const int     f = tid / 18, n = (tid % 18) / 3, c = tid % 3, h = f >> 1, w = f & 1;
+        const int     fr = 2 * rc + (h >> 2);
+        const double  r0 = A.radii[fr], r1 = A.radii[fr + 1];
+        const double  rm = 0.5 * (r0 + r1), hdr = 0.5 * (r1 - r0);
+        const double  alpha = 0.5 / rm, beta = 1.0 / (6.0 * hdr);
+        const double* gw = column(h) + 10 * w;
+        const double  L  = n % 3 == 0 ? -(gw[c] + gw[3 + c]) : (n % 3 == 1 ? gw[c] : gw[3 + c]);
+        G[f][n][c]       = alpha * L + (n < 3 ? -beta : beta) * gw[6 + c];
+    } else if (tid < kFineWedges * 19) {
+        const int f = tid - kFineWedges * 18, h = f >> 1, w = f & 1;
+        int       fx, fy, fr;
+        fine_hex(h, xc, yc, rc, fx, fy, fr);
+        const double r0 = A.radii[fr], r1 = A.radii[fr + 1];
+        const double rm = 0.5 * (r0 + r1), hdr = 0.5 * (r1 - r0);
+        double       kv;
+        if (A.kq0) {
+            kv = A.kq0[node_index(nlf - 1, nrf - 1, d, fx, fy, fr)];
+        } else {
+            const double wlat0 = 1.0 - 1.0 / 3.0 - 1.0 / 3.0, wlat = 1.0 / 3.0;
+            kv                 = 0.0;
+            for (int n = 0; n < 6; ++n)
+                kv += (n % 3 == 0 ? wlat0 : wlat) * 0.5 *
+                      A.k[node_index(nlf, nrf, d, fx + woff(w, n, 0), fy + woff(w, n, 1), fr + woff(w, n, 2))];
+        }
+        kw[f] = kv * column(h)[10 * w + 9] * rm * rm * hdr;
+    } else if (tid < kFineWedges * 25) {
+        const int f = (tid - kFineWedges * 19) / 6, fl = (tid - kFineWedges * 19) % 6;
+        int       fx, fy, fr;
+        fine_hex(f >> 1, xc, yc, rc, fx, fy, fr);
+        interp_row(d, fx, fy, fr, f & 1, fl, nlf, nrf, A.linw, P[f][fl]);
+    }
+    __syncthreads();
+    if (tid < kFineWedges * 18) {
+        const int f = tid / 18, c = (tid % 18) / 3, a = tid % 3;
+        double    h = 0.0;
+#pragma unroll
+        for (int n = 0; n < 6; ++n) h += P[f][n][c] * G[f][n][a];
+        H[f][c][a] = h;
+    }
+    __syncthreads();
+    if (tid >= 2 * kPack) return;
+    const int t = tid / kPack, p = tid % kPack;
+    int       i, j;
+    packed_pair(p, i, j);
+    const int ni = i % 6, di = i / 6, nj = j % 6, dj = j / 6;
+    double    acc = 0.0;
+    for (int f = 0; f < kFineWedges; ++f) {
+        if (target_wedge(f >> 1, f & 1) != t) continue;
+        const double* hi = H[f][ni];
+        const double* hj = H[f][nj];
+        double        v  = hi[dj] * hj[di] - (2.0 / 3.0) * hi[di] * hj[dj];
+        if (di == dj) v += hi[0] * hj[0] + hi[1] * hj[1] + hi[2] * hj[2];
+        acc += kw[f] * v;
+    }
+    A.out[static_cast<int64_t>(t * kPack + p) * A.nout + slot] = acc;
+}
+
 // Element matrices of one level itself (no coarsening): the stored form of the
 // on-the-fly operator (get_local_matrix of a level without stored matrices).
 // Slot s of out holds cell cells[s] (or s); with base given, out = base - A_e
@@ -1150,7 +1233,10 @@ int gca_build(int nlf, int nrf, const double* coords_f, const double* radii_f, c
     } else if (fine_mats == nullptr) {
         if (!colgeo_f || build_smem_configure() != 0) return -1;
         a.colgeo = colgeo_f;
-        gca_build_rank_kernel<<<(a.nout + kRankCells - 1) / kRankCells, 32 * kRankWarps, kRankSmem, st>>>(a);
+        if (a.nout <= (a.linw ? kHexCellsLinear : kHexCells))
+            gca_build_hex_kernel<<<a.nout, kHexThreads, 0, st>>>(a);
+        else
+            gca_build_rank_kernel<<<(a.nout + kRankCells - 1) / kRankCells, 32 * kRankWarps, kRankSmem, st>>>(a);
     } else {
         if (build_smem_configure() != 0) return -1;
         gca_build_mma_kernel<<<a.nout, kMmaThreads, kMmaSmem, st>>>(a);

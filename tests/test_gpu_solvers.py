@@ -636,12 +636,13 @@ def test_compact_store_fp32(cuda, lat, rad, nlev, bcs):
     assert ((out[1] - out[0]).norm() / out[0].norm()).item() < 4e-6
 
 
-@pytest.mark.parametrize("lat,rad", [(1, 2), (2, 2), (2, 3), (3, 2)])
+@pytest.mark.parametrize("lat,rad", [(1, 2), (2, 2), (2, 3), (3, 2), (4, 2), (4, 3), (4, 4)])
 @pytest.mark.parametrize("q0", [False, True])
 @pytest.mark.parametrize("interpolation", [0, 1])
 def test_fast_gca_build_equals_plain_build(cuda, lat, rad, q0, interpolation):
-    """The build over on-the-fly matrices, 32 coarse hexes a block, against the plain one on cell counts that do not fill
-    the last block and with one or several radial layers; the two round differently in the last bits (1e-13)."""
+    """The build over on-the-fly matrices against the plain one, with one or several radial layers: a coarse hex a block up
+    to 1024 of them (2560 for linear interpolation; the levels listed have 20 to 320, 1280, 2560 and 5120), 32 hexes a
+    block above. The two round differently in the last bits (1e-13)."""
     g = T.Shell(lat, rad, num_levels=2)
     nl, nr = g.dims(1)
     nlc, nrc = g.dims(0)
@@ -653,6 +654,30 @@ def test_fast_gca_build_equals_plain_build(cuda, lat, rad, q0, interpolation):
     for fast in (True, False):
         coarse = T.EpsDivDiv(g, 0, k=_t(np.ones((10, nlc, nlc, nrc))))
         T.gca_build(fine, coarse, interpolation=interpolation, tensor_cores=fast)
+        mats.append(coarse.local_matrices())
+    assert rel_err(mats[0], mats[1]) < 1e-13
+
+
+@pytest.mark.parametrize("cells", [1, 1024, 1025, 1537, 2561])
+@pytest.mark.parametrize("interpolation", [0, 1])
+def test_fast_gca_build_of_listed_cells(cuda, cells, interpolation):
+    """The same over a list of cells: counts on both sides of the lines, and such that do not fill the last block of 32."""
+    import torch
+
+    g = T.Shell(4, num_levels=2)
+    nl, nr = g.dims(1)
+    nlc, nrc = g.dims(0)
+    rng = np.random.default_rng(cells)
+    fine = T.EpsDivDiv(g, 1, k=_t(np.exp(rng.uniform(-2.0, 2.0, (10, nl, nl, nr)))))
+    marks = np.zeros(10 * (nlc - 1) ** 2 * (nrc - 1), np.uint8)
+    marks[rng.permutation(marks.size)[:cells]] = 1
+    marks = torch.tensor(marks.reshape(10, nlc - 1, nlc - 1, nrc - 1), device=cuda)
+    mats = []
+    for fast in (True, False):
+        coarse = T.EpsDivDiv(g, 0, k=_t(np.ones((10, nlc, nlc, nrc))))
+        coarse.set_selective_matrices(0, marks)
+        T.gca_build(fine, coarse, interpolation=interpolation, tensor_cores=fast)
+        assert coarse.stored_cells()[0] == cells
         mats.append(coarse.local_matrices())
     assert rel_err(mats[0], mats[1]) < 1e-13
 
