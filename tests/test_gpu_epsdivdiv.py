@@ -231,3 +231,31 @@ def test_chained_applies_equal_synchronised(cuda, level):
         torch.cuda.synchronize()
         out.append(u)
     assert torch.isfinite(out[0]).all() and torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("lat,rad", [(0, 1), (1, 1), (2, 3), (3, 1), (1, 6)])
+@pytest.mark.parametrize("bcs", [(0, 0), (1, 2), (2, 2), (2, 0)])
+@pytest.mark.parametrize("q0", [False, True])
+def test_diagonal_shapes(cuda, lat, rad, bcs, q0):
+    """Diagonal mode on levels of two radial layers and many, both coefficients, with and without free-slip nodes (a launch
+    of their own), replacing and adding: FP64 1e-12 as above, FP32 1e-5 (sums of 12 terms at 6e-8)."""
+    import torch
+
+    sh, gsh = O.Shell(lat, rad), T.Shell(lat, rad)
+    rng = np.random.default_rng(lat + 10 * rad)
+    k = np.exp(rng.uniform(-1.0, 1.0, sh.cell_shape)) if q0 else smooth_viscosity(sh, 12, 50.0)
+    u = O.seeded_normal(sh.vec_shape, 13)
+    ref = O.EpsDivDiv(sh, **({"k_q0": k} if q0 else {"k": k}), bc_cmb=bcs[0], bc_surface=bcs[1]).apply(
+        u, path="slow", diagonal=True)
+    for dt, tol in ((torch.float64, 1e-12), (torch.float32, 1e-5)):
+        kt, ut = (torch.tensor(a, dtype=dt, device=cuda) for a in (k, u))
+        op = T.EpsDivDiv(gsh, **({"k_cell": kt} if q0 else {"k": kt}), bc_cmb=bcs[0], bc_surface=bcs[1], diagonal=True)
+        out = torch.zeros_like(ut)
+        op.apply(ut, out)
+        assert rel_err(out.double().cpu().numpy(), ref) < tol
+        op.set_modes(T.ADD, T.SKIP_COMMUNICATION)
+        once = torch.zeros_like(ut)
+        op.apply(ut, once)
+        twice = once.clone()
+        op.apply(ut, twice)
+        assert torch.equal(twice, 2 * once)
